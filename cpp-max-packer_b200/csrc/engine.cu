@@ -405,6 +405,46 @@ int greedy_step(spk_context* ctx, Session& s, const std::vector<std::size_t>& su
     for (std::size_t o = 0; o < O; ++o) {
         exhausted[o] = !active[o];
     }
+    const auto request = [&](std::size_t o) {
+        PageRequest r;
+        r.slot = s.slot_of[o];
+        r.has_cursor = cursors[o].has_value();
+        if (r.has_cursor) {
+            r.cursor = *cursors[o];
+        }
+        return r;
+    };
+    // Certified pages for `which`, in place of those orientations' heads.
+    const auto resolve = [&](const std::vector<std::size_t>& which) {
+        std::vector<PageRequest> requests;
+        for (std::size_t o : which) {
+            requests.push_back(request(o));
+        }
+        std::vector<PageOutcome> out;
+        int status = session_pages(ctx, s, requests, out, { true, true });
+        if (status) {
+            return status;
+        }
+        for (std::size_t k = 0; k < which.size(); ++k) {
+            if (out[k].status) {
+                return out[k].status;
+            }
+            const auto o = which[k];
+            pages[o] = std::move(out[k].page);
+            index[o] = 0;
+            floor[o] = out[k].page.size() == static_cast<std::size_t>(kPageSize) || !out[k].certified
+                           ? out[k].exact_floor
+                           : INFINITY;
+            if (out[k].certified && floor[o] < INFINITY && !pages[o].empty()) {
+                floor[o] = std::max(floor[o], pages[o].back().score);
+            }
+            loaded[o] = true;
+            if (pages[o].empty()) {
+                exhausted[o] = true;
+            }
+        }
+        return static_cast<int>(kOk);
+    };
     for (;;) {
         // (Re)load pages that are consumed: lazily, all at once.
         std::vector<PageRequest> requests;
@@ -417,13 +457,7 @@ int greedy_step(spk_context* ctx, Session& s, const std::vector<std::size_t>& su
                 exhausted[o] = true;  // a complete page was fully consumed
                 continue;
             }
-            PageRequest r;
-            r.slot = s.slot_of[o];
-            r.has_cursor = cursors[o].has_value();
-            if (r.has_cursor) {
-                r.cursor = *cursors[o];
-            }
-            requests.push_back(r);
+            requests.push_back(request(o));
             which.push_back(o);
         }
         if (!requests.empty()) {
@@ -445,13 +479,30 @@ int greedy_step(spk_context* ctx, Session& s, const std::vector<std::size_t>& su
                     exhausted[o] = true;
                 }
             }
-            // Widen while too few active orientations admit a copy.
+            // Widen while too few active orientations admit a copy.  An empty
+            // page decides that only where the orientation is exhausted: heads
+            // leave out the planes above the best head's bound, and a copy may
+            // fit there.
             if (next_reserve < reserve.size() && block > 0) {
-                std::size_t feasible = 0;
-                for (std::size_t o = 0; o < O; ++o) {
-                    feasible += active[o] && !pages[o].empty() ? 1 : 0;
+                const auto feasible = [&] {
+                    std::size_t n = 0;
+                    for (std::size_t o = 0; o < O; ++o) {
+                        n += active[o] && !pages[o].empty() ? 1 : 0;
+                    }
+                    return n;
+                };
+                if (feasible() < min_feasible) {
+                    std::vector<std::size_t> undecided;
+                    for (std::size_t o = 0; o < O; ++o) {
+                        if (active[o] && !exhausted[o] && pages[o].empty()) {
+                            undecided.push_back(o);
+                        }
+                    }
+                    if (!undecided.empty() && (status = resolve(undecided))) {
+                        return status;
+                    }
                 }
-                if (feasible < min_feasible) {
+                if (feasible() < min_feasible) {
                     for (std::size_t added = 0; added < block && next_reserve < reserve.size(); ++next_reserve) {
                         const std::size_t o = reserve[next_reserve];
                         if (o < O && !active[o]) {
@@ -479,8 +530,7 @@ int greedy_step(spk_context* ctx, Session& s, const std::vector<std::size_t>& su
             }
         }
         // Orientations whose next exact candidate could precede it.
-        std::vector<PageRequest> resolve;
-        std::vector<std::size_t> resolve_which;
+        std::vector<std::size_t> inexact;
         for (std::size_t o = 0; o < O; ++o) {
             if (exhausted[o]) {
                 continue;
@@ -496,38 +546,11 @@ int greedy_step(spk_context* ctx, Session& s, const std::vector<std::size_t>& su
             if (best && lower > pages[*best][index[*best]].score) {
                 continue;
             }
-            PageRequest r;
-            r.slot = s.slot_of[o];
-            r.has_cursor = cursors[o].has_value();
-            if (r.has_cursor) {
-                r.cursor = *cursors[o];
-            }
-            resolve.push_back(r);
-            resolve_which.push_back(o);
+            inexact.push_back(o);
         }
-        if (!resolve.empty()) {
-            std::vector<PageOutcome> out;
-            int status = session_pages(ctx, s, resolve, out, { true, true });
-            if (status) {
+        if (!inexact.empty()) {
+            if (int status = resolve(inexact)) {
                 return status;
-            }
-            for (std::size_t k = 0; k < resolve_which.size(); ++k) {
-                if (out[k].status) {
-                    return out[k].status;
-                }
-                const auto o = resolve_which[k];
-                pages[o] = std::move(out[k].page);
-                index[o] = 0;
-                floor[o] = out[k].page.size() == static_cast<std::size_t>(kPageSize) || !out[k].certified
-                               ? out[k].exact_floor
-                               : INFINITY;
-                if (out[k].certified && floor[o] < INFINITY && !pages[o].empty()) {
-                    floor[o] = std::max(floor[o], pages[o].back().score);
-                }
-                loaded[o] = true;
-                if (pages[o].empty()) {
-                    exhausted[o] = true;
-                }
             }
             continue;
         }

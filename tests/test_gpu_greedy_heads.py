@@ -1,0 +1,56 @@
+"""The greedy's pruned heads: an orientation whose free planes lie above the
+best head's bound comes back with an empty page whose planes above were not
+visited.  Such a page says nothing about them, so it must not count as
+"admits no copy".
+
+The scene is a narrow tower of plates: flat items fit into every gap from the
+floor up, upright ones only above the top plate, far past the bound of the
+best flat head."""
+
+import numpy as np
+import pytest
+
+from conftest import package
+from oracle import proposal_net
+
+pytestmark = pytest.mark.gpu
+
+HALF = 2 ** -0.5
+# Flat twice (identity, half a turn about z), upright twice (a quarter about x and y).
+CATALOG = np.array([[0, 0, 0, 1], [0, 0, 1, 0], [HALF, 0, 0, HALF], [0, HALF, 0, HALF]], np.float64)
+FLAT, UPRIGHT = (0, 1), (2, 3)
+
+
+def _tower(ctx, top):
+    """A 16 x 16 x 180 box with plates every nine cells up to `top`."""
+    assets, session_mod, synthetic = package("assets"), package("session"), package("synthetic")
+    item = assets.accept_stl(synthetic.cuboid_stl((14.0, 14.0, 4.0)))
+    s = session_mod.Session(item, (16.0, 16.0, 180.0), (0.0, 0.0, 0.0), 1.0, CATALOG, context=ctx)
+    x, y, z = min((c.translation for c in s.pages([0])[0]), key=lambda t: t[2])
+    for above in range(9, top, 9):
+        s.place(0, (x, y, z + above))
+    return s
+
+
+def _net(ctx):
+    net = package("proposal").Proposal(context=ctx)
+    net.set_parameters(proposal_net.he_parameters(9).astype(np.float32))
+    return net
+
+
+@pytest.mark.parametrize("top,upright_fits", [(150, True), (176, False)])
+def test_widening_counts_orientations_that_are_free_high_up(gpu_ctx, top, upright_fits):
+    proposal = package("proposal")
+    s = _tower(gpu_ctx, top)
+    fits = [bool(page) for page in s.pages(range(4))]  # whole pages
+    assert fits == [True, True, upright_fits, upright_fits]
+    best = s.greedy(1)[0]
+    s.remove_last()
+    net = _net(gpu_ctx)
+    # Any three of the four hold a flat and an upright one.
+    placed, fallbacks, widenings = proposal.greedy_proposed_adaptive(s, net, 3, 3, 1)
+    assert widenings == (0 if upright_fits else 1)
+    assert fallbacks == 0
+    assert placed[0].score == best.score
+    net.close()
+    s.close()
