@@ -446,7 +446,9 @@ int greedy_step(spk_context* ctx, Session& s, const std::vector<std::size_t>& su
         return static_cast<int>(kOk);
     };
     for (;;) {
-        // (Re)load pages that are consumed: lazily, all at once.
+        // (Re)load pages that are consumed: lazily, all at once.  An empty page
+        // with a finite floor had no entry to consume: its orientation waits until
+        // the floor could precede the best entry, and is resolved then.
         std::vector<PageRequest> requests;
         std::vector<std::size_t> which;
         for (std::size_t o = 0; o < O; ++o) {
@@ -455,6 +457,9 @@ int greedy_step(spk_context* ctx, Session& s, const std::vector<std::size_t>& su
             }
             if (loaded[o] && floor[o] == INFINITY) {
                 exhausted[o] = true;  // a complete page was fully consumed
+                continue;
+            }
+            if (loaded[o] && pages[o].empty()) {
                 continue;
             }
             requests.push_back(request(o));
@@ -519,17 +524,23 @@ int greedy_step(spk_context* ctx, Session& s, const std::vector<std::size_t>& su
                 next_reserve = reserve.size();  // enough feasible orientations: no more widening
             }
         }
-        // Best exact head.
+        // Best exact head, and the lowest score of any: every entry is a
+        // candidate with its exact score, so nothing above that is chosen next.
         std::optional<std::size_t> best;
+        double bound = INFINITY;
         for (std::size_t o = 0; o < O; ++o) {
-            if (exhausted[o] || index[o] >= pages[o].size() || pages[o][index[o]].score > floor[o]) {
+            if (exhausted[o] || index[o] >= pages[o].size()) {
+                continue;
+            }
+            bound = std::min(bound, pages[o][index[o]].score);
+            if (pages[o][index[o]].score > floor[o]) {
                 continue;
             }
             if (!best || rank_less(pages[o][index[o]], pages[*best][index[*best]])) {
                 best = o;
             }
         }
-        // Orientations whose next exact candidate could precede it.
+        // Orientations whose next exact candidate could be the choice.
         std::vector<std::size_t> inexact;
         for (std::size_t o = 0; o < O; ++o) {
             if (exhausted[o]) {
@@ -543,7 +554,7 @@ int greedy_step(spk_context* ctx, Session& s, const std::vector<std::size_t>& su
             if (index[o] < pages[o].size()) {
                 lower = std::min(lower, pages[o][index[o]].score);
             }
-            if (best && lower > pages[*best][index[*best]].score) {
+            if (lower > bound) {
                 continue;
             }
             inexact.push_back(o);
