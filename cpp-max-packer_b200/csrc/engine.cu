@@ -432,7 +432,8 @@ int greedy_step(spk_context* ctx, Session& s, const std::vector<std::size_t>& su
             const auto o = which[k];
             pages[o] = std::move(out[k].page);
             index[o] = 0;
-            floor[o] = out[k].page.size() == static_cast<std::size_t>(kPageSize) || !out[k].certified
+            // A certified page that is not full holds every candidate there is.
+            floor[o] = pages[o].size() == static_cast<std::size_t>(kPageSize) || !out[k].certified
                            ? out[k].exact_floor
                            : INFINITY;
             if (out[k].certified && floor[o] < INFINITY && !pages[o].empty()) {

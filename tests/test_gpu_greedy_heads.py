@@ -5,7 +5,8 @@ copy", and the orientation need not be paged again until its floor could win.
 
 The scene is a narrow tower of plates: flat items fit into every gap from the
 floor up, upright ones only above the top plate, far past the bound of the
-best flat head."""
+best flat head.  The last test walks a fill through several pages of one
+orientation."""
 
 import numpy as np
 import pytest
@@ -85,3 +86,27 @@ def test_rejected_poses_page_undecided_orientations_only_when_they_could_win(gpu
     else:
         # Their floors are reached at some rejection; a whole page settles them.
         assert paged <= flat_alone + 2 * len(UPRIGHT)
+
+
+def test_rejections_walk_through_more_than_one_page(gpu_ctx):
+    assets, session_mod, synthetic = package("assets"), package("session"), package("synthetic")
+    item = assets.accept_stl(synthetic.cuboid_stl((9.0, 7.0, 5.0)))
+    s = session_mod.Session(item, (24.0, 22.0, 20.0), (0.0, 0.0, 0.0), 1.0, CATALOG[:1], context=gpu_ctx)
+    want, cursor = [], None
+    while len(want) < 81:  # three pages of 32, each after the one before
+        page = s.pages([0], cursors=[cursor])[0]
+        assert len(page) == 32
+        want += [c.translation for c in page]
+        cursor = page[-1]
+    seen = []
+
+    def validate(_orientation, translation, _pose, _q):
+        seen.append(translation)
+        return len(seen) > 80
+
+    s.set_validator(validate)
+    placed = s.greedy(1)
+    s.set_validator(None)
+    s.close()
+    assert seen == want[:81]
+    assert [p.translation for p in placed] == want[80:81]
