@@ -1232,16 +1232,6 @@ int Pipeline::low_overlap_page(const PageRequest& req, PageOutcome& out)
     return kOk;
 }
 
-// The FP32 bound of a count's residual is far from reached: over 3,700 pages
-// (windows of 66 to 256 cells, items of 3,000 to 80,000) no residual came to more
-// than 1/31 of it.  Where the bound lies in [0.25, kWatchedEpsilon) a request is
-// pruned as long as its visited planes' residuals stay within kQuietResidual, a
-// quarter of the guard; otherwise it is computed again over all planes.
-// (Heads of 96 orientations of 29,000 to 48,000 cells on a 128^3 window, bounds
-// of 0.3 to 0.4: a step takes 1.60 ms without pruning, 0.90 ms with it.)
-constexpr double kWatchedEpsilon = 1.0;
-constexpr float kQuietResidual = 0.0625f;
-
 int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vector<PageOutcome>& out, PageGoal goal)
 {
     const int R = static_cast<int>(requests.size());
@@ -1257,7 +1247,6 @@ int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vect
         double eps {}, floor {};
         double prune_key { INFINITY }, prune_exact { INFINITY };
         int z {}, end {};  // legal planes [z, end) are still to be visited
-        bool watched {}, unpruned {};  // the residual decides on pruning; it decided against
     };
     std::vector<Lane> lanes(R);
     std::vector<int> runnable;
@@ -1278,12 +1267,10 @@ int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vect
         l.eps = approx_epsilon(s) + std::ldexp(1.0, -22);
         l.floor = requests[r].has_cursor ? requests[r].cursor.score - l.eps : -INFINITY;
         l.end = s.legal[2];
-        // Planes are pruned only where every count's residual keeps inside the
-        // guard: a residual beyond it must be seen wherever it is.  Below
-        // 0.25 the FP32 bound says so.  Up to kWatchedEpsilon the visited
-        // planes' residual has to say so too.
-        if (goal.prune && requests[r].overlap == 0 && epsilon_p(s) < kWatchedEpsilon) {
-            l.watched = epsilon_p(s) >= 0.25;
+        // Planes are pruned only where the FP32 bound keeps every count's
+        // residual inside the guard: one beyond it must be seen wherever it is,
+        // and the planes that were visited say nothing about the others.
+        if (goal.prune && requests[r].overlap == 0 && epsilon_p(s) < 0.25) {
             const double occ = static_cast<double>(s.occupied);
             feasible_planes(s, l.z, l.end);
             l.prune_exact = .35 * s.most_proximity / occ + 1e-12;
@@ -1440,10 +1427,6 @@ int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vect
             float rf;
             std::memcpy(&rf, &rbits, 4);
             o.max_integer_residual = rf;
-            if (lanes[r].watched && rf > kQuietResidual) {
-                lanes[r].unpruned = true;
-                continue;
-            }
             if (rf >= 0.25f) {
                 o.status = kNumeric;  // correlation.cpp:521-528 residual guard
                 continue;
@@ -1538,7 +1521,7 @@ int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vect
             }
             for (int r : runnable) {
                 const Lane& l = lanes[r];
-                if (!out[r].status && !l.unpruned && l.z < l.end && l.s->t65_host[l.z] - l.prune_exact <= best) {
+                if (!out[r].status && l.z < l.end && l.s->t65_host[l.z] - l.prune_exact <= best) {
                     again.push_back(r);
                 }
             }
@@ -1546,14 +1529,7 @@ int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vect
         active = std::move(again);
         step = step > INT32_MAX / 2 ? INT32_MAX : 2 * step;
     }
-    std::vector<PageRequest> whole;
-    std::vector<int> whole_of;
     for (int r : runnable) {
-        if (lanes[r].unpruned) {
-            whole.push_back(requests[r]);
-            whole_of.push_back(r);
-            continue;
-        }
         if (!out[r].status) {
             ++stat_pages;
             stat_first_certified += out[r].certified ? 1 : 0;
@@ -1565,7 +1541,7 @@ int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vect
     // rescore all of them exactly, and widen T until the page is certified.
     for (int r = 0; r < R && goal.full; ++r) {
         auto& o = out[r];
-        if (o.status || o.certified || lanes[r].unpruned) {
+        if (o.status || o.certified) {
             continue;
         }
         const auto& req = requests[r];
@@ -1672,15 +1648,6 @@ int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vect
         }
         if (!o.certified && !o.status) {
             o.status = kScratchLimit;
-        }
-    }
-    if (!whole.empty()) {
-        std::vector<PageOutcome> again;
-        if ((status = ordinary_pages(whole, again, { goal.full, false }))) {
-            return status;
-        }
-        for (std::size_t k = 0; k < whole_of.size(); ++k) {
-            out[whole_of[k]] = std::move(again[k]);
         }
     }
     return kOk;
