@@ -1041,7 +1041,7 @@ int spk_session_open(spk_context* ctx, const spk_session_desc* d, spk_session_in
                                       s->origin, s->pitch, s->wall, s->mask))) {
             return status;
         }
-        s->pipe = std::make_unique<Pipeline>(ctx);
+        s->pipe = std::make_unique<Pipeline>(ctx, "pipe");
         if ((status = s->pipe->set_geometry(s->env.first, s->env.shape, s->origin, s->pitch, s->cmin_z, s->height))) {
             return status;
         }

@@ -25,7 +25,7 @@ extern "C" int spk_spectral_page(spk_context* ctx, const spk_page_scene* scene, 
         if (cudaSetDevice(ctx->device) != cudaSuccess) {
             return kCuda;
         }
-        Pipeline pipe(ctx);
+        Pipeline pipe(ctx, "page.pipe");
         int status = pipe.set_geometry(scene->environment_first, scene->environment_shape, scene->lattice_origin_mm,
                                        scene->lattice_pitch_mm, scene->container_min_z_mm,
                                        scene->container_height_mm);

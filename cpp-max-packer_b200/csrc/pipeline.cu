@@ -516,7 +516,7 @@ bool rank_less(const Candidate& l, const Candidate& r)
 
 }  // namespace
 
-Pipeline::Pipeline(spk_context* ctx) : ctx_(ctx)
+Pipeline::Pipeline(spk_context* ctx, const char* name) : ctx_(ctx), name_(name)
 {
     const char* fixed = std::getenv("SPK_FFT_LENGTHS");
     pow2_ = fixed && std::strcmp(fixed, "pow2") == 0;
@@ -580,13 +580,14 @@ int Pipeline::set_geometry(const std::int64_t* env_first, const std::uint32_t* e
     const long long grid = static_cast<long long>(L_[0]) * L_[1] * E_[2];
     const std::size_t row_blocks = static_cast<std::size_t>((E_[1] + kRowsPerBlock - 1) / kRowsPerBlock) * E_[2];
     int status = kOk;
-    occ_ = static_cast<std::uint8_t*>(device_buffer(ctx_, "pipe.occ", cells, status));
-    d2_ = static_cast<std::int32_t*>(device_buffer(ctx_, "pipe.d2", cells * sizeof(std::int32_t), status));
-    env_ = static_cast<float2*>(device_buffer(ctx_, "pipe.env", grid * sizeof(float2), status));
-    stats_ = static_cast<RowStats*>(device_buffer(ctx_, "pipe.stats", row_blocks * sizeof(RowStats), status));
+    occ_ = static_cast<std::uint8_t*>(device_buffer(ctx_, name_ + ".occ", cells, status));
+    d2_ = static_cast<std::int32_t*>(device_buffer(ctx_, name_ + ".d2", cells * sizeof(std::int32_t), status));
+    env_ = static_cast<float2*>(device_buffer(ctx_, name_ + ".env", grid * sizeof(float2), status));
+    stats_ = static_cast<RowStats*>(device_buffer(ctx_, name_ + ".stats", row_blocks * sizeof(RowStats), status));
     const long long tiles = static_cast<long long>((E_[0] + kEdtTile - 1) / kEdtTile) *
                             ((E_[1] + kEdtTile - 1) / kEdtTile) * ((E_[2] + kEdtTile - 1) / kEdtTile);
-    tile_max_ = static_cast<std::int32_t*>(device_buffer(ctx_, "pipe.tile_max", tiles * sizeof(std::int32_t), status));
+    tile_max_ =
+        static_cast<std::int32_t*>(device_buffer(ctx_, name_ + ".tile_max", tiles * sizeof(std::int32_t), status));
     if (!occ_ || !d2_ || !env_ || !stats_ || !tile_max_) {
         return status;
     }
@@ -594,8 +595,14 @@ int Pipeline::set_geometry(const std::int64_t* env_first, const std::uint32_t* e
     if (!proximity_shape_supported(shape)) {
         return kProximityShape;
     }
-    table_ = proximity_table(ctx_, max_squared_distance(shape), status);
-    return table_ ? kOk : status;
+    return table(status) ? kOk : status;
+}
+
+const double* Pipeline::table(int& status) const
+{
+    const std::uint32_t shape[3] = { static_cast<std::uint32_t>(E_[0]), static_cast<std::uint32_t>(E_[1]),
+                                     static_cast<std::uint32_t>(E_[2]) };
+    return proximity_table(ctx_, max_squared_distance(shape), status);
 }
 
 int Pipeline::set_occupancy(const std::uint8_t* d_occupancy)
@@ -637,10 +644,11 @@ int Pipeline::update_spectrum(const EdtBox* d_region)
     int status = kOk;
     const auto* tw0 = twiddle_table<float>(ctx_, L_[0], status);
     const auto* tw1 = twiddle_table<float>(ctx_, L_[1], status);
-    if (!tw0 || !tw1) {
+    const double* proximity = table(status);
+    if (!tw0 || !tw1 || !proximity) {
         return status;
     }
-    if (launch_env_rows(L_[0], L_[1], env_, E_, occ_, d2_, table_, tw0, stats_, d_region, st) != cudaSuccess ||
+    if (launch_env_rows(L_[0], L_[1], env_, E_, occ_, d2_, proximity, tw0, stats_, d_region, st) != cudaSuccess ||
         launch_forward_y(L_[0], L_[1], env_, E_[1], E_[2], tw1, d_region, st) != cudaSuccess) {
         cudaGetLastError();
         return kCuda;
@@ -650,7 +658,7 @@ int Pipeline::update_spectrum(const EdtBox* d_region)
     // (finish_stats) only when a page needs them, so nothing here waits.
     const std::size_t bytes =
         sizeof(RowStats) * static_cast<std::size_t>((E_[1] + kRowsPerBlock - 1) / kRowsPerBlock) * E_[2];
-    auto* host = static_cast<RowStats*>(host_buffer(ctx_, "pipe.stats", bytes, status));
+    auto* host = static_cast<RowStats*>(host_buffer(ctx_, name_ + ".stats", bytes, status));
     if (!host) {
         return status;
     }
@@ -816,7 +824,8 @@ int Pipeline::add_kernels(std::uint64_t first_orientation, const std::vector<geo
         auto* h_result = static_cast<char*>(host_buffer(ctx_, "pipe.kernel_result", result_bytes, status));
         const auto* tw0 = twiddle_table<float>(ctx_, L_[0], status);
         const auto* tw1 = twiddle_table<float>(ctx_, L_[1], status);
-        if (!h_table || !d_table || !depth || !d_result || !h_result || !tw0 || !tw1) {
+        const double* proximity = table(status);
+        if (!h_table || !d_table || !depth || !d_result || !h_result || !tw0 || !tw1 || !proximity) {
             return status;
         }
         std::memcpy(h_table, items.data(), items_bytes);
@@ -852,7 +861,7 @@ int Pipeline::add_kernels(std::uint64_t first_orientation, const std::vector<geo
         depth_pass_kernel<<<grid, 128, 0, st>>>(d_items, d_cells, nullptr, depth, 0);
         depth_pass_kernel<<<grid, 128, 0, st>>>(d_items, d_cells, depth, depth + total, 1);
         depth_pass_kernel<<<grid, 128, 0, st>>>(d_items, d_cells, depth + total, depth, 2);
-        depth_plane_kernel<<<static_cast<unsigned>(planes), 256, 0, st>>>(d_items, d_plane_item, depth, table_,
+        depth_plane_kernel<<<static_cast<unsigned>(planes), 256, 0, st>>>(d_items, d_plane_item, depth, proximity,
                                                                          d_planes);
         ctx_->launches += 7;
         cudaMemcpyAsync(h_result, d_result, result_bytes, cudaMemcpyDeviceToHost, st);
@@ -1314,7 +1323,8 @@ int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vect
     const std::size_t job_bytes = R * sizeof(ExactJob);
     auto* d_jobs = static_cast<char*>(device_buffer(ctx_, "pipe.jobs", job_bytes + R * sizeof(int), status));
     auto* h_jobs = static_cast<char*>(host_buffer(ctx_, "pipe.jobs", job_bytes + R * sizeof(int), status));
-    if (!partial || !result || !host || !d_jobs || !h_jobs) {
+    const double* proximity = table(status);
+    if (!partial || !result || !host || !d_jobs || !h_jobs || !proximity) {
         return status;
     }
     unsigned long long* tau = result;
@@ -1401,8 +1411,8 @@ int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vect
             merge_lists_kernel<<<n, 64, 0, st>>>(partial, d_lanes, static_cast<int>(chunks), per, selected);
             ctx_->launches++;
         }
-        exact_kernel<<<n * exact, kExactThreads, 0, st>>>(selected, jobs, d_lanes, per, exact, occ_, d2_, table_, E_[0],
-                                                          E_[1], counts_out, p_out, range_error);
+        exact_kernel<<<n * exact, kExactThreads, 0, st>>>(selected, jobs, d_lanes, per, exact, occ_, d2_, proximity,
+                                                          E_[0], E_[1], counts_out, p_out, range_error);
         pass_end(ctx_, 3, ev);
         ctx_->launches += 2;
         cudaMemcpyAsync(host, result, words * 8, cudaMemcpyDeviceToHost, st);
@@ -1592,8 +1602,8 @@ int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vect
                     return status;
                 }
                 exact_kernel<<<n, kExactThreads, 0, st>>>(tkeys, jobs + r, nullptr, static_cast<int>(n),
-                                                          static_cast<int>(n), occ_, d2_, table_, E_[0], E_[1], tcount,
-                                                          tp, range_error);
+                                                          static_cast<int>(n), occ_, d2_, proximity, E_[0], E_[1],
+                                                          tcount, tp, range_error);
                 ctx_->launches++;
                 std::vector<unsigned long long> hk(n);
                 std::vector<long long> cnt(n);

@@ -15,6 +15,7 @@
 
 #include <cmath>
 #include <cstdint>
+#include <string>
 #include <vector>
 
 #include "../../include/spk_b200.h"
@@ -101,7 +102,9 @@ constexpr int kHeadCandidates = 16;
 
 class Pipeline {
 public:
-    explicit Pipeline(spk_context* ctx);
+    // `name` prefixes the context's buffers that hold this pipeline's state
+    // between calls: pipelines that live side by side need different ones.
+    Pipeline(spk_context* ctx, const char* name);
     ~Pipeline();
 
     // Environment window (global first + shape) and lattice/container terms.
@@ -166,10 +169,13 @@ private:
     int finish_stats();
     // Transform lengths per axis for the window; sets L_.
     int choose_lengths(const std::uint32_t* env_shape);
+    // The proximity table, which other calls on the context may have moved.
+    const double* table(int& status) const;
     double score(const KernelSlot& s, const std::int64_t* t, double p) const;
     double approx_epsilon(const KernelSlot& s) const;
 
     spk_context* ctx_;
+    const std::string name_;
     int E_[3] {};
     int L_[3] {};  // x and y transform lengths; z: the length a whole column would take
     bool pow2_ {};   // SPK_FFT_LENGTHS=pow2
@@ -183,7 +189,6 @@ private:
     std::int32_t* d2_ {};
     std::int32_t* tile_max_ {};  // largest d2 per kEdtTile^3 tile (incremental EDT)
     float2* env_ {};             // [z < E2][ky < L1][kx < L0]: Z = B + iP, x and y transformed
-    const double* table_ {};
     RowStats* stats_ {};             // device, one entry per row block
     const RowStats* stats_host_ {};  // pinned copy of the last update
     cudaStream_t stats_stream_ {};
