@@ -602,7 +602,10 @@ const double* Pipeline::table(int& status) const
 {
     const std::uint32_t shape[3] = { static_cast<std::uint32_t>(E_[0]), static_cast<std::uint32_t>(E_[1]),
                                      static_cast<std::uint32_t>(E_[2]) };
-    return proximity_table(ctx_, max_squared_distance(shape), status);
+    // A kernel cell lies at most as deep as half its window's shortest side and
+    // one, within the window's largest distance except in a window of one cell,
+    // whose kernel is one cell deep.
+    return proximity_table(ctx_, std::max(max_squared_distance(shape), 1), status);
 }
 
 int Pipeline::set_occupancy(const std::uint8_t* d_occupancy)
