@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <string>
@@ -74,6 +75,19 @@ inline void* device_buffer(spk_context* ctx, const std::string& name, std::size_
     b.bytes = bytes;
     ctx->bytes_in_use += bytes;
     return p;
+}
+
+// Gives named device buffers back.
+inline void drop_buffers(spk_context* ctx, std::initializer_list<const char*> names)
+{
+    for (const char* name : names) {
+        const auto it = ctx->device_buffers.find(name);
+        if (it != ctx->device_buffers.end()) {
+            cudaFree(it->second.ptr);
+            ctx->bytes_in_use -= it->second.bytes;
+            ctx->device_buffers.erase(it);
+        }
+    }
 }
 
 // A device block of at least `bytes` (set to its size) for an object that gives

@@ -1045,23 +1045,42 @@ int spk_session_open(spk_context* ctx, const spk_session_desc* d, spk_session_in
         if ((status = s->pipe->set_geometry(s->env.first, s->env.shape, s->origin, s->pitch, s->cmin_z, s->height))) {
             return status;
         }
-        // Orientations in batches of bounded scratch (72 bytes of intervals
-        // per vertex).
+        // Orientations in batches of bounded scratch: 256 MB of intervals (72
+        // bytes per vertex) and kBatchCells cells.  Where even that is more than
+        // the context may have, or the device has left, in smaller batches down
+        // to one orientation at a time.
+        const auto drop_scratch = [&] {
+            drop_buffers(ctx, { "field.vint", "field.pose_bounds", "field.poses", "field.items", "field.parent",
+                                "field.rootv", "obj.cells", "pipe.depth", "pipe.kernel_table", "pipe.kernel_result" });
+        };
         const std::size_t O = s->catalog.size();
-        const std::size_t per = std::max<std::size_t>(
+        std::size_t per = std::max<std::size_t>(
             1, std::min<std::size_t>(64, (256ULL << 20) / (s->object_mesh.vertices.size() * sizeof(IVec3))));
-        for (std::size_t o = 0; o < O; o += per) {
+        for (std::size_t o = 0; o < O;) {
             const int n = static_cast<int>(std::min(per, O - o));
             ObjectFields fields;
-            if ((status = object_fields(ctx, s->object, s->object_tris, s->object_vertices, s->origin, s->pitch,
-                                        s->catalog.data() + o, n, fields)) ||
-                (status = s->pipe->add_kernels(o, fields.windows, fields.d_cells, fields.cells_at.data(),
-                                               fields.max_z.data()))) {
+            if (!(status = object_fields(ctx, s->object, s->object_tris, s->object_vertices, s->origin, s->pitch,
+                                         s->catalog.data() + o, n, fields))) {
+                if (ctx->cap_bytes) {
+                    drop_buffers(ctx, { "field.vint", "field.misc" });  // of the raster alone
+                }
+                status = s->pipe->add_kernels(o, fields.windows, fields.d_cells, fields.cells_at.data(),
+                                              fields.max_z.data());
+            }
+            if ((status == kMemoryLimit || status == kAllocation) && n > 1) {
+                drop_scratch();
+                per = n / 2;
+                continue;
+            }
+            if (status) {
                 return status;
             }
-            for (int i = 0; i < n; ++i) {
-                s->slot_of.push_back(o + i);
+            for (std::size_t i = 0; i < fields.windows.size(); ++i) {
+                s->slot_of.push_back(o++);
             }
+        }
+        if (ctx->cap_bytes) {
+            drop_scratch();  // under a cap, what a batch needed is wanted elsewhere
         }
         ctx->session = s.release();
         return spk_session_info_get(ctx, info);

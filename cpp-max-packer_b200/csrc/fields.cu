@@ -643,16 +643,16 @@ int raster_batch(spk_context* ctx, const RasterBatch& b, std::uint8_t* d_cells, 
     }
     const int F = static_cast<int>(b.mesh->triangles.size()), V = static_cast<int>(b.mesh->vertices.size());
     int status = kOk;
-    const unsigned int root_capacity = 1u << 20;
+    const auto root_capacity = static_cast<unsigned int>(ctx->cap_bytes ? std::min(total, 1LL << 20) : 1LL << 20);
     constexpr unsigned int kEarlyRoots = 240;  // read back with the flags
     auto* d_parent = static_cast<int*>(device_buffer(ctx, "field.parent", total * sizeof(int), status));
-    auto* d_rootv = static_cast<std::uint8_t*>(device_buffer(ctx, "field.rootv", total, status));
     // [0] errors, [1] roots found, from [16] on the roots.
-    auto* d_misc = static_cast<int*>(device_buffer(ctx, "field.misc", (16 + root_capacity) * 4ULL, status));
+    auto* d_misc = static_cast<int*>(device_buffer(
+        ctx, "field.misc", (16 + std::max(root_capacity, kEarlyRoots)) * 4ULL, status));
     auto* h_misc = static_cast<int*>(host_buffer(ctx, "field.misc", (16 + kEarlyRoots) * 4ULL, status));
     RasterItem single {};
     RasterItem* d_items = nullptr;
-    if (!d_parent || !d_rootv || !d_misc || !h_misc) {
+    if (!d_parent || !d_misc || !h_misc) {
         return status;
     }
     long long largest = 1, rows = 1;
@@ -796,6 +796,7 @@ int raster_batch(spk_context* ctx, const RasterBatch& b, std::uint8_t* d_cells, 
         return kFieldIndexOverflow;
     }
     FewRoots few {};
+    std::uint8_t* d_rootv = nullptr;
     few.count = roots <= static_cast<unsigned>(kFewRoots) ? static_cast<int>(roots) : -1;
     for (int k = 0; k < few.count; ++k) {
         few.root[k] = h_roots[k];
@@ -804,7 +805,8 @@ int raster_batch(spk_context* ctx, const RasterBatch& b, std::uint8_t* d_cells, 
     if (few.count < 0) {
         auto* h_values = static_cast<std::uint8_t*>(host_buffer(ctx, "field.values", roots, status));
         auto* d_values = static_cast<std::uint8_t*>(device_buffer(ctx, "field.values", roots, status));
-        if (!h_values || !d_values) {
+        d_rootv = static_cast<std::uint8_t*>(device_buffer(ctx, "field.rootv", total, status));
+        if (!h_values || !d_values || !d_rootv) {
             return status;
         }
         std::memcpy(h_values, values.data(), roots);
@@ -974,9 +976,9 @@ int object_fields(spk_context* ctx, const geo::Prepared& prepared, const std::ui
     const geo::Vec3 translation { origin[0], origin[1], origin[2] };
     cudaStream_t st = ctx->stream;
     int status = kOk;
-    out.windows.assign(count, {});
-    out.max_z.assign(count, 0.0);
-    out.cells_at.assign(count + 1, 0);
+    out.windows.clear();
+    out.max_z.clear();
+    out.cells_at.assign(1, 0);
     auto* d_vint = static_cast<IVec3*>(
         device_buffer(ctx, "field.vint", static_cast<std::size_t>(count) * V * sizeof(IVec3), status));
     if (!d_vint) {
@@ -986,59 +988,59 @@ int object_fields(spk_context* ctx, const geo::Prepared& prepared, const std::ui
     if ((status = device_intervals(ctx, mesh, d_vertices, translation, q, count, true, d_vint, bounds))) {
         return status;
     }
-    std::vector<geo::Placed> placed(count);
-    std::vector<FieldWindow> windows(count);
+    std::vector<geo::Placed> placed;
+    std::vector<FieldWindow> windows;
     std::vector<int> on_host;
-    for (int i = 0; i < count; ++i) {
+    int taken = 0;
+    for (; taken < count; ++taken) {
+        const int i = taken;
+        geo::Placed pose;
+        geo::Window window;
+        double max_z = 0;
+        bool host = false;
         if (!geo::canonical_unit(q[i])) {
             return kFieldInput;
         }
         std::optional<geo::RotationTransform> transform;
         if (device_pose(translation, q[i], transform) && !bounds[i].invalid && !bounds[i].oriented_invalid) {
-            placed[i] = device_placed(prepared, translation, q[i], *transform, bounds[i]);
-            out.max_z[i] = bounds[i].oriented_hi(2);
+            pose = device_placed(prepared, translation, q[i], *transform, bounds[i]);
+            max_z = bounds[i].oriented_hi(2);
         }
         else {
             geo::Bounds oriented;
-            if (!geo::place(prepared, translation, q[i], placed[i]) || !geo::oriented_bounds(mesh, q[i], oriented)) {
+            if (!geo::place(prepared, translation, q[i], pose) || !geo::oriented_bounds(mesh, q[i], oriented)) {
                 return kFieldInput;
             }
-            out.max_z[i] = oriented.max[2];
-            on_host.push_back(i);
+            max_z = oriented.max[2];
+            host = true;
         }
-        if (!geo::object_window(placed[i], origin, pitch, out.windows[i])) {
+        if (!geo::object_window(pose, origin, pitch, window)) {
             return kFieldIndexOverflow;
         }
-        windows[i] = make_window(out.windows[i], origin, pitch);
-        out.cells_at[i + 1] = out.cells_at[i] + window_cells(windows[i]);
+        const FieldWindow w = make_window(window, origin, pitch);
+        const long long end = out.cells_at[i] + window_cells(w);
+        if (i > 0 && end > kBatchCells) {
+            break;
+        }
+        if (host) {
+            on_host.push_back(i);
+        }
+        placed.push_back(std::move(pose));
+        windows.push_back(w);
+        out.windows.push_back(window);
+        out.max_z.push_back(max_z);
+        out.cells_at.push_back(end);
     }
     for (int i : on_host) {
         cudaMemcpyAsync(d_vint + static_cast<long long>(i) * V, placed[i].intervals.data(), V * sizeof(IVec3),
                         cudaMemcpyHostToDevice, st);
     }
-    out.d_cells = static_cast<std::uint8_t*>(device_buffer(ctx, "obj.cells", out.cells_at[count], status));
+    out.d_cells = static_cast<std::uint8_t*>(device_buffer(ctx, "obj.cells", out.cells_at[taken], status));
     if (!out.d_cells) {
         return status;
     }
-    // Batches of bounded size: labels take four bytes per cell.
-    constexpr long long kBatchCells = 64LL << 20;
-    for (int i0 = 0; i0 < count;) {
-        int i1 = i0 + 1;
-        while (i1 < count && out.cells_at[i1 + 1] - out.cells_at[i0] <= kBatchCells) {
-            ++i1;
-        }
-        std::vector<long long> cells_at(out.cells_at.begin() + i0, out.cells_at.begin() + i1 + 1);
-        for (auto& at : cells_at) {
-            at -= out.cells_at[i0];
-        }
-        const RasterBatch batch { &mesh, placed.data() + i0, windows.data() + i0, i1 - i0, cells_at.data(), d_tris,
-                                  d_vint + static_cast<long long>(i0) * V };
-        if ((status = raster_batch(ctx, batch, out.d_cells + out.cells_at[i0], true, false))) {
-            return status;
-        }
-        i0 = i1;
-    }
-    return kOk;
+    return raster_batch(ctx, { &mesh, placed.data(), windows.data(), taken, out.cells_at.data(), d_tris, d_vint },
+                        out.d_cells, true, false);
 }
 
 int dilate_crop(spk_context* ctx, const std::uint8_t* d_raw, const FieldWindow& raw, std::uint64_t halo,

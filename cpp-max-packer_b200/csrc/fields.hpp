@@ -39,14 +39,20 @@ inline FieldWindow make_window(const geo::Window& w, const double* origin, doubl
 int raster_fill(spk_context* ctx, const geo::Placed& placed, const FieldWindow& w, std::uint8_t* d_cells,
                 bool normalize, const std::uint32_t* d_tris_kept = nullptr, bool device_intervals = false);
 
-// voxelize_object (conservative_fields.cpp:919-1003) for `count` rotations of
-// one mesh at once: windows, the cells of all on the device (0/1, item i at
+// voxelize_object (conservative_fields.cpp:919-1003) for the first of `count`
+// rotations of one mesh, as many as fit kBatchCells cells of their windows, at
+// least one: windows, the cells of all on the device (0/1, item i at
 // d_cells + cells_at[i], in a context buffer that the next call reuses) and
 // the oriented bounds' max z.  The work is queued on the context's stream.
+//
+// A batch takes about 14 bytes of scratch per cell on the device (cells,
+// labels, roots, depths).  16 M cells hold 64 orientations of 60^3 windows;
+// whole waves of blocks come from far fewer.
+constexpr long long kBatchCells = 16LL << 20;
 struct ObjectFields {
-    std::vector<geo::Window> windows;
+    std::vector<geo::Window> windows;  // of the rotations taken
     std::vector<double> max_z;
-    std::vector<long long> cells_at;  // count + 1 entries
+    std::vector<long long> cells_at;  // one more entry
     std::uint8_t* d_cells {};
 };
 int object_fields(spk_context* ctx, const geo::Prepared& prepared, const std::uint32_t* d_tris,

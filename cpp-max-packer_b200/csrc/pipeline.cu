@@ -297,6 +297,7 @@ __device__ __forceinline__ unsigned long long warp_merge(unsigned long long a, u
 // in only batches that can change them, and the warps' sets are merged in
 // pairs.  The result is that of the two-stage merge, which sorts whole chunks
 // for longer lists (96 requests: 18 and 7 us for its kernels, 5.3 us this way).
+constexpr int kFewKeys = 32;
 constexpr int kHeadThreads = 1024;
 __global__ void __launch_bounds__(kHeadThreads) merge_heads_kernel(const unsigned long long* __restrict__ keys,
                                                                   unsigned int cap,
@@ -804,6 +805,27 @@ int Pipeline::add_kernels(std::uint64_t first_orientation, const std::vector<geo
         for (int i : fit) {
             t65_count += slots[i].t65_host.size();
         }
+        // Tables of the batch, up in one copy: items, planes' items, .65 top.
+        const std::size_t items_bytes = items.size() * sizeof(KernelItem);
+        const std::size_t table_bytes = (items_bytes + planes * sizeof(int) + 7) / 8 * 8;
+        auto* h_table = static_cast<char*>(
+            host_buffer(ctx_, "pipe.kernel_table", table_bytes + t65_count * sizeof(double), status));
+        auto* d_table = static_cast<char*>(device_buffer(ctx_, "pipe.kernel_table", table_bytes, status));
+        // The passes of the depths alternate between a buffer and the raster's
+        // labels, which are done with.
+        const std::size_t depth_bytes = total * sizeof(std::int32_t);
+        auto* depth = static_cast<std::int32_t*>(device_buffer(ctx_, "pipe.depth", depth_bytes, status));
+        auto* other = static_cast<std::int32_t*>(device_buffer(ctx_, "field.parent", depth_bytes, status));
+        // Results: plane statistics, then counts.
+        const std::size_t result_bytes = planes * sizeof(RowStats) + fit.size() * sizeof(unsigned int);
+        auto* d_result = static_cast<char*>(device_buffer(ctx_, "pipe.kernel_result", result_bytes, status));
+        auto* h_result = static_cast<char*>(host_buffer(ctx_, "pipe.kernel_result", result_bytes, status));
+        const auto* tw0 = twiddle_table<float>(ctx_, L_[0], status);
+        const auto* tw1 = twiddle_table<float>(ctx_, L_[1], status);
+        const double* proximity = table(status);
+        if (!h_table || !d_table || !depth || !other || !d_result || !h_result || !tw0 || !tw1 || !proximity) {
+            return status;
+        }
         Block block { nullptr, partial_bytes + ones_bytes + t65_count * sizeof(double) };
         block.ptr = take_block(ctx_, block.bytes, status);
         if (!block.ptr) {
@@ -813,24 +835,6 @@ int Pipeline::add_kernels(std::uint64_t first_orientation, const std::vector<geo
         auto* partial = static_cast<float2*>(block.ptr);
         auto* ones = reinterpret_cast<std::int32_t*>(static_cast<char*>(block.ptr) + partial_bytes);
         auto* t65 = reinterpret_cast<double*>(reinterpret_cast<char*>(ones) + ones_bytes);
-        // Tables of the batch, up in one copy: items, planes' items, .65 top.
-        const std::size_t items_bytes = items.size() * sizeof(KernelItem);
-        const std::size_t table_bytes = (items_bytes + planes * sizeof(int) + 7) / 8 * 8;
-        auto* h_table = static_cast<char*>(
-            host_buffer(ctx_, "pipe.kernel_table", table_bytes + t65_count * sizeof(double), status));
-        auto* d_table = static_cast<char*>(device_buffer(ctx_, "pipe.kernel_table", table_bytes, status));
-        auto* depth = static_cast<std::int32_t*>(
-            device_buffer(ctx_, "pipe.depth", 2 * total * sizeof(std::int32_t), status));
-        // Results: plane statistics, then counts.
-        const std::size_t result_bytes = planes * sizeof(RowStats) + fit.size() * sizeof(unsigned int);
-        auto* d_result = static_cast<char*>(device_buffer(ctx_, "pipe.kernel_result", result_bytes, status));
-        auto* h_result = static_cast<char*>(host_buffer(ctx_, "pipe.kernel_result", result_bytes, status));
-        const auto* tw0 = twiddle_table<float>(ctx_, L_[0], status);
-        const auto* tw1 = twiddle_table<float>(ctx_, L_[1], status);
-        const double* proximity = table(status);
-        if (!h_table || !d_table || !depth || !d_result || !h_result || !tw0 || !tw1 || !proximity) {
-            return status;
-        }
         std::memcpy(h_table, items.data(), items_bytes);
         std::memcpy(h_table + items_bytes, plane_item.data(), planes * sizeof(int));
         auto* h_t65 = reinterpret_cast<double*>(h_table + table_bytes);
@@ -862,8 +866,8 @@ int Pipeline::add_kernels(std::uint64_t first_orientation, const std::vector<geo
             return kCuda;
         }
         depth_pass_kernel<<<grid, 128, 0, st>>>(d_items, d_cells, nullptr, depth, 0);
-        depth_pass_kernel<<<grid, 128, 0, st>>>(d_items, d_cells, depth, depth + total, 1);
-        depth_pass_kernel<<<grid, 128, 0, st>>>(d_items, d_cells, depth + total, depth, 2);
+        depth_pass_kernel<<<grid, 128, 0, st>>>(d_items, d_cells, depth, other, 1);
+        depth_pass_kernel<<<grid, 128, 0, st>>>(d_items, d_cells, other, depth, 2);
         depth_plane_kernel<<<static_cast<unsigned>(planes), 256, 0, st>>>(d_items, d_plane_item, depth, proximity,
                                                                          d_planes);
         ctx_->launches += 7;
@@ -1024,6 +1028,11 @@ int Pipeline::run_planes(const std::vector<PlaneWork>& work, PassMode mode, bool
             const std::size_t bytes = plane_cells * W * sizeof(float2);
             int per_launch = static_cast<int>(
                 std::min<std::size_t>(std::max<std::size_t>(kInterBytes / bytes, 1), static_cast<std::size_t>(n)));
+            if (ctx_->cap_bytes) {  // half of what is left: placements need theirs
+                const std::uint64_t left = ctx_->cap_bytes - ctx_->bytes_in_use;
+                per_launch = static_cast<int>(
+                    std::max<std::uint64_t>(1, std::min<std::uint64_t>(per_launch, left / 2 / bytes)));
+            }
             float2* inter = nullptr;
             while (!inter) {  // under a device-memory cap, fewer orientations per launch
                 inter = static_cast<float2*>(device_buffer(ctx_, "pipe.inter", bytes * per_launch, status));
@@ -1262,7 +1271,7 @@ int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vect
     };
     std::vector<Lane> lanes(R);
     std::vector<int> runnable;
-    int deepest = 1;
+    int deepest = 1, most_planes = 1;
     long long most_blocks = 1;
     for (int r = 0; r < R; ++r) {
         const auto& s = slots_[requests[r].slot];
@@ -1290,6 +1299,7 @@ int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vect
             l.prune_key = .35 * (s.most_proximity + 2 * epsilon_p(s)) / occ + 4e-7;
         }
         deepest = std::max(deepest, s.K[2]);
+        most_planes = std::max(most_planes, s.legal[2]);
         most_blocks = std::max(most_blocks, (static_cast<long long>(s.legal[1]) * s.legal[2] + 15) / 16);
         runnable.push_back(r);
     }
@@ -1304,19 +1314,6 @@ int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vect
     const int per = exact + 1;
     unsigned int chunks = static_cast<unsigned int>(std::min<long long>(
         kMaxKeyChunks, std::max<long long>(1, (most_blocks * 64 + kKeyCapacity - 1) / kKeyCapacity)));
-    unsigned long long* keys = nullptr;
-    while (!keys) {  // under a device-memory cap, a shorter range that may overflow
-        keys = static_cast<unsigned long long*>(
-            device_buffer(ctx_, "pipe.keys", static_cast<std::size_t>(R) * chunks * kKeyCapacity * 8, status));
-        if (!keys && chunks == 1) {
-            return status;
-        }
-        chunks = keys ? chunks : chunks / 2;
-    }
-    status = kOk;
-    const unsigned int cap = chunks * kKeyCapacity;
-    auto* partial = static_cast<unsigned long long*>(
-        device_buffer(ctx_, "pipe.partial", static_cast<std::size_t>(R) * chunks * per * 8, status));
     // One result block, read back in one copy: bound, residual and key count
     // per request, then per candidate its key, exact count and exact sum, then
     // the range flag.
@@ -1327,9 +1324,38 @@ int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vect
     auto* d_jobs = static_cast<char*>(device_buffer(ctx_, "pipe.jobs", job_bytes + R * sizeof(int), status));
     auto* h_jobs = static_cast<char*>(host_buffer(ctx_, "pipe.jobs", job_bytes + R * sizeof(int), status));
     const double* proximity = table(status);
-    if (!partial || !result || !host || !d_jobs || !h_jobs || !proximity) {
+    if (!result || !host || !d_jobs || !h_jobs || !proximity) {
         return status;
     }
+    if (ctx_->cap_bytes) {
+        // One orientation's intermediate comes first (run_planes takes room for
+        // more where there is some), then keys in up to a quarter of what is left:
+        // a shorter range, which may overflow.
+        if (!device_buffer(ctx_, "pipe.inter", sizeof(float2) * L_[0] * L_[1] * most_planes, status)) {
+            return status;
+        }
+        const std::uint64_t chunk_bytes = static_cast<std::uint64_t>(R) * (kKeyCapacity + per) * 8;
+        while (chunks > 1 && chunks * chunk_bytes > (ctx_->cap_bytes - ctx_->bytes_in_use) / 4) {
+            chunks /= 2;
+        }
+    }
+    // The first stage's winners (the heads' merge has one stage).
+    unsigned long long* partial = nullptr;
+    if (per > kFewKeys && !(partial = static_cast<unsigned long long*>(device_buffer(
+                                ctx_, "pipe.partial", static_cast<std::size_t>(R) * chunks * per * 8, status)))) {
+        return status;
+    }
+    unsigned long long* keys = nullptr;
+    while (!keys) {  // where memory is short, a shorter range as well
+        keys = static_cast<unsigned long long*>(
+            device_buffer(ctx_, "pipe.keys", static_cast<std::size_t>(R) * chunks * kKeyCapacity * 8, status));
+        if (!keys && chunks == 1) {
+            return status;
+        }
+        chunks = keys ? chunks : chunks / 2;
+    }
+    status = kOk;
+    const unsigned int cap = chunks * kKeyCapacity;
     unsigned long long* tau = result;
     unsigned long long* resid = tau + R;
     unsigned long long* count = resid + R;
@@ -1405,7 +1431,7 @@ int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vect
         first = false;
         const int n = static_cast<int>(active.size());
         auto ev = pass_begin(ctx_);
-        if (per <= 32) {
+        if (per <= kFewKeys) {
             merge_heads_kernel<<<n, kHeadThreads, 0, st>>>(keys, cap, count, d_lanes, per, selected);
         }
         else {
