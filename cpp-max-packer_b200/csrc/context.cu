@@ -58,9 +58,7 @@ void spk_context_destroy(spk_context* ctx)
     for (auto e : ctx->copy_events) {
         cudaEventDestroy(e);
     }
-    for (auto& b : ctx->kept_blocks) {
-        cudaFree(b.ptr);
-    }
+    spk::release_kept_blocks(ctx);
     for (auto& [key, p] : ctx->twiddles) {
         cudaFree(p);
     }

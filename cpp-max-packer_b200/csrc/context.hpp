@@ -31,7 +31,8 @@ struct spk_context {
     std::map<std::string, Buffer> device_buffers;
     std::map<std::string, Buffer> host_buffers;  // pinned staging
     // Device blocks given back by sessions for the next one to take
-    // (take_block, give_block): at most kKeptBytes of them.
+    // (take_block, give_block): at most kKeptBytes of them, within the cap, and
+    // only as long as nothing else on the context needs the memory.
     static constexpr std::size_t kKeptBytes = 256ULL << 20;
     std::vector<Buffer> kept_blocks;
     std::vector<cudaEvent_t> copy_events;  // one per pinned copy slot (host_copy.cu)
@@ -48,7 +49,47 @@ struct spk_context {
 
 namespace spk {
 
+inline std::uint64_t kept_bytes(const spk_context* ctx)
+{
+    std::uint64_t sum = 0;
+    for (const auto& b : ctx->kept_blocks) {
+        sum += b.bytes;
+    }
+    return sum;
+}
+
+inline void release_kept_blocks(spk_context* ctx)
+{
+    for (const auto& b : ctx->kept_blocks) {
+        cudaFree(b.ptr);
+    }
+    ctx->kept_blocks.clear();
+}
+
+// Device memory; the blocks kept for the next session go where there is none
+// left.  nullptr on failure.
+inline void* device_alloc(spk_context* ctx, std::size_t bytes)
+{
+    void* p {};
+    if (cudaMalloc(&p, bytes ? bytes : 1) == cudaSuccess) {
+        return p;
+    }
+    cudaGetLastError();
+    if (ctx->kept_blocks.empty()) {
+        return nullptr;
+    }
+    release_kept_blocks(ctx);
+    if (cudaMalloc(&p, bytes ? bytes : 1) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return p;
+}
+
 // Grows (never shrinks) a named device buffer; returns nullptr on failure.
+// These buffers are what the context's cap is about; blocks kept for the next
+// session take no room from it, and go where both would exceed it.  (An open
+// session's kernel data, take_block, lies outside the cap.)
 inline void* device_buffer(spk_context* ctx, const std::string& name, std::size_t bytes, int& status)
 {
     auto& b = ctx->device_buffers[name];
@@ -60,14 +101,16 @@ inline void* device_buffer(spk_context* ctx, const std::string& name, std::size_
         status = kMemoryLimit;
         return nullptr;
     }
+    if (ctx->cap_bytes && next + kept_bytes(ctx) > ctx->cap_bytes) {
+        release_kept_blocks(ctx);
+    }
     if (b.ptr) {
         cudaFree(b.ptr);
         ctx->bytes_in_use -= b.bytes;
         b = {};
     }
-    void* p {};
-    if (cudaMalloc(&p, bytes ? bytes : 1) != cudaSuccess) {
-        cudaGetLastError();
+    void* p = device_alloc(ctx, bytes);
+    if (!p) {
         status = kAllocation;
         return nullptr;
     }
@@ -110,30 +153,17 @@ inline void* take_block(spk_context* ctx, std::size_t& bytes, int& status)
         ctx->kept_blocks.erase(best);
         return p;
     }
-    void* p {};
-    if (cudaMalloc(&p, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        // The kept blocks may be what is missing.
-        for (auto& b : ctx->kept_blocks) {
-            cudaFree(b.ptr);
-        }
-        ctx->kept_blocks.clear();
-        if (cudaMalloc(&p, bytes) != cudaSuccess) {
-            cudaGetLastError();
-            status = kAllocation;
-            return nullptr;
-        }
+    void* p = device_alloc(ctx, bytes);
+    if (!p) {
+        status = kAllocation;
     }
     return p;
 }
 
 inline void give_block(spk_context* ctx, void* ptr, std::size_t bytes)
 {
-    std::size_t kept = bytes;
-    for (const auto& b : ctx->kept_blocks) {
-        kept += b.bytes;
-    }
-    if (kept > spk_context::kKeptBytes) {
+    const std::uint64_t kept = kept_bytes(ctx) + bytes;
+    if (kept > spk_context::kKeptBytes || (ctx->cap_bytes && ctx->bytes_in_use + kept > ctx->cap_bytes)) {
         cudaFree(ptr);
         return;
     }
@@ -204,9 +234,8 @@ const cplx_t<T>* twiddle_table(spk_context* ctx, int L, int& status)
         host[m].x = static_cast<T>(c);
         host[m].y = static_cast<T>(s);
     }
-    void* p {};
-    if (cudaMalloc(&p, sizeof(cplx_t<T>) * L) != cudaSuccess) {
-        cudaGetLastError();
+    void* p = device_alloc(ctx, sizeof(cplx_t<T>) * L);
+    if (!p) {
         status = kAllocation;
         return nullptr;
     }

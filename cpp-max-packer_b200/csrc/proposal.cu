@@ -1199,11 +1199,10 @@ constexpr bool shapes_have_gradients()
 static_assert(shapes_have_gradients(), "strides, channel and voxel counts that the gradients are written for");
 
 template <typename T>
-int alloc(ProposalNet* net, T*& p, std::size_t count)
+int alloc(spk_context* ctx, ProposalNet* net, T*& p, std::size_t count)
 {
-    void* raw {};
-    if (cudaMalloc(&raw, sizeof(T) * (count ? count : 1)) != cudaSuccess) {
-        cudaGetLastError();
+    void* raw = device_alloc(ctx, sizeof(T) * count);
+    if (!raw) {
         return kAllocation;
     }
     net->owned.push_back(raw);
@@ -1222,7 +1221,7 @@ void release(ProposalNet* net, T*& p)
     p = nullptr;
 }
 
-int ensure_batch(ProposalNet* net, std::uint32_t batch)
+int ensure_batch(spk_context* ctx, ProposalNet* net, std::uint32_t batch)
 {
     if (batch <= net->capacity) {
         return kOk;
@@ -1238,20 +1237,20 @@ int ensure_batch(ProposalNet* net, std::uint32_t batch)
     release(net, net->dpred);
     release(net, net->loss_terms);
     net->capacity = 0;
-    int s = alloc(net, net->x0, static_cast<std::size_t>(batch) * kProposalVoxels * 2);
+    int s = alloc(ctx, net, net->x0, static_cast<std::size_t>(batch) * kProposalVoxels * 2);
     for (int l = 0; l < kProposalLayers && !s; ++l) {
         const int so = out_side(kProposalSpec[l]);
         const std::size_t n = static_cast<std::size_t>(batch) * so * so * so * kProposalSpec[l].cout;
-        s = alloc(net, net->act[l], n);
+        s = alloc(ctx, net, net->act[l], n);
         if (!s) {
-            s = alloc(net, net->dpre[l], n);
+            s = alloc(ctx, net, net->dpre[l], n);
         }
     }
-    if (!s) s = alloc(net, net->pred, batch);
-    if (!s) s = alloc(net, net->labels, batch);
-    if (!s) s = alloc(net, net->pooled, static_cast<std::size_t>(batch) * 64);
-    if (!s) s = alloc(net, net->dpred, batch);
-    if (!s) s = alloc(net, net->loss_terms, batch);
+    if (!s) s = alloc(ctx, net, net->pred, batch);
+    if (!s) s = alloc(ctx, net, net->labels, batch);
+    if (!s) s = alloc(ctx, net, net->pooled, static_cast<std::size_t>(batch) * 64);
+    if (!s) s = alloc(ctx, net, net->dpred, batch);
+    if (!s) s = alloc(ctx, net, net->loss_terms, batch);
     if (s) {
         return s;
     }
@@ -1261,14 +1260,14 @@ int ensure_batch(ProposalNet* net, std::uint32_t batch)
 
 // Grows a device buffer to at least `count` elements (contents discarded).
 template <typename T>
-int reserve(ProposalNet* net, T*& p, std::size_t& capacity, std::size_t count)
+int reserve(spk_context* ctx, ProposalNet* net, T*& p, std::size_t& capacity, std::size_t count)
 {
     if (p && count <= capacity) {
         return kOk;
     }
     release(net, p);
     capacity = 0;
-    if (int status = alloc(net, p, count)) {
+    if (int status = alloc(ctx, net, p, count)) {
         return status;
     }
     capacity = count;
@@ -1391,7 +1390,7 @@ int launch_gradients(spk_context* ctx, ProposalNet* net, std::uint32_t batch)
             if (need > net->partial_bytes) {
                 release(net, net->partial);
                 net->partial_bytes = 0;
-                if ((status = alloc(net, net->partial, need / sizeof(float)))) {
+                if ((status = alloc(ctx, net, net->partial, need / sizeof(float)))) {
                     return status;
                 }
                 net->partial_bytes = need;
@@ -1519,7 +1518,7 @@ int predict_box(spk_context* ctx, ProposalNet* net, std::uint32_t batch, const b
     int status = kOk;
     if (net->item_half_tag != items_tag || net->item_half_batch != batch || net->item_half_version != net->version ||
         !net->item_half_box) {
-        if (!net->support && (status = alloc(net, net->support, 3))) {
+        if (!net->support && (status = alloc(ctx, net, net->support, 3))) {
             return status;
         }
         cudaMemsetAsync(net->support, 0, 3 * sizeof(unsigned), ctx->stream);
@@ -1544,8 +1543,8 @@ int predict_box(spk_context* ctx, ProposalNet* net, std::uint32_t batch, const b
         }
         const std::size_t item_vol = static_cast<std::size_t>(net->item_box[0]) * net->item_box[1] * net->item_box[2];
         const std::size_t vol0 = static_cast<std::size_t>(net->box[0][0]) * net->box[0][1] * net->box[0][2];
-        if ((status = reserve(net, net->x_item, net->x_item_capacity, batch * item_vol * 2)) ||
-            (status = reserve(net, net->item_half, net->item_half_capacity, batch * vol0 * c1))) {
+        if ((status = reserve(ctx, net, net->x_item, net->x_item_capacity, batch * item_vol * 2)) ||
+            (status = reserve(ctx, net, net->item_half, net->item_half_capacity, batch * vol0 * c1))) {
             return status;
         }
         if (item_vol) {
@@ -1562,24 +1561,24 @@ int predict_box(spk_context* ctx, ProposalNet* net, std::uint32_t batch, const b
         net->item_half_box = true;
         net->trunk_valid = false;
     }
-    if ((!net->x_crop && (status = alloc(net, net->x_crop, static_cast<std::size_t>(kProposalVoxels) * 2))) ||
-        (!net->crop_half && (status = alloc(net, net->crop_half, static_cast<std::size_t>(kProposalVoxels) * c1))) ||
-        (!net->prev_crop && (status = alloc(net, net->prev_crop, static_cast<std::size_t>(kProposalVoxels)))) ||
-        (!net->dirty && (status = alloc(net, net->dirty, 6)))) {
+    if ((!net->x_crop && (status = alloc(ctx, net, net->x_crop, static_cast<std::size_t>(kProposalVoxels) * 2))) ||
+        (!net->crop_half && (status = alloc(ctx, net, net->crop_half, static_cast<std::size_t>(kProposalVoxels) * c1))) ||
+        (!net->prev_crop && (status = alloc(ctx, net, net->prev_crop, static_cast<std::size_t>(kProposalVoxels)))) ||
+        (!net->dirty && (status = alloc(ctx, net, net->dirty, 6)))) {
         return status;
     }
     for (int l = 0; l < kProposalLayers; ++l) {
         const ProposalLayer& L = kProposalSpec[l];
         const std::size_t so = static_cast<std::size_t>(out_side(L));
         const std::size_t vol = static_cast<std::size_t>(net->box[l][0]) * net->box[l][1] * net->box[l][2];
-        if ((!net->act_shared[l] && (status = alloc(net, net->act_shared[l], so * so * so * L.cout))) ||
-            (status = reserve(net, net->act_box[l], net->act_box_capacity[l], batch * vol * L.cout))) {
+        if ((!net->act_shared[l] && (status = alloc(ctx, net, net->act_shared[l], so * so * so * L.cout))) ||
+            (status = reserve(ctx, net, net->act_box[l], net->act_box_capacity[l], batch * vol * L.cout))) {
             return status;
         }
     }
     const int s3 = out_side(kProposalSpec[kProposalLayers - 1]);
     const int c3 = kProposalSpec[kProposalLayers - 1].cout;
-    if ((status = reserve(net, net->box_last, net->box_last_capacity,
+    if ((status = reserve(ctx, net, net->box_last, net->box_last_capacity,
                           static_cast<std::size_t>(batch) * s3 * s3 * s3 * c3))) {
         return status;
     }
@@ -1719,7 +1718,7 @@ int proposal_predict(spk_context* ctx, ProposalNet* net, std::uint32_t batch, co
     if (!crop_index && !item_index && crops && items && items_tag && !full_trunk()) {
         return predict_box(ctx, net, batch, crops, items, items_tag, pred);
     }
-    int status = ensure_batch(net, batch);
+    int status = ensure_batch(ctx, net, batch);
     if (status) {
         return status;
     }
@@ -1736,7 +1735,7 @@ int proposal_predict(spk_context* ctx, ProposalNet* net, std::uint32_t batch, co
             if (half > net->item_half_capacity) {
                 release(net, net->item_half);
                 net->item_half_capacity = 0;
-                if ((status = alloc(net, net->item_half, half))) {
+                if ((status = alloc(ctx, net, net->item_half, half))) {
                     return status;
                 }
                 net->item_half_capacity = half;
@@ -1750,7 +1749,7 @@ int proposal_predict(spk_context* ctx, ProposalNet* net, std::uint32_t batch, co
             net->item_half_version = net->version;
             net->item_half_box = false;
         }
-        if (!net->crop_half && (status = alloc(net, net->crop_half, static_cast<std::size_t>(kProposalVoxels) * c1))) {
+        if (!net->crop_half && (status = alloc(ctx, net, net->crop_half, static_cast<std::size_t>(kProposalVoxels) * c1))) {
             return status;
         }
         assemble_kernel<<<grid_for(kProposalVoxels), 256, 0, ctx->stream>>>(crops, nullptr, nullptr, nullptr, 1,
@@ -1878,15 +1877,15 @@ int spk_proposal_create(spk_context* ctx, uint64_t seed, spk_proposal** out)
         }
         off += 64;
         net->head_b = off;
-        int s = spk::alloc(net, net->params, net->count);
-        if (!s) s = spk::alloc(net, net->grads, net->count);
-        if (!s) s = spk::alloc(net, net->adam_m, net->count);
-        if (!s) s = spk::alloc(net, net->adam_v, net->count);
-        if (!s) s = spk::alloc(net, net->loss, 1);
-        if (!s) s = spk::alloc(net, net->error, 1);
+        int s = spk::alloc(ctx, net, net->params, net->count);
+        if (!s) s = spk::alloc(ctx, net, net->grads, net->count);
+        if (!s) s = spk::alloc(ctx, net, net->adam_m, net->count);
+        if (!s) s = spk::alloc(ctx, net, net->adam_v, net->count);
+        if (!s) s = spk::alloc(ctx, net, net->loss, 1);
+        if (!s) s = spk::alloc(ctx, net, net->error, 1);
         for (int l = 0; l < spk::kProposalLayers && !s; ++l) {
             const spk::ProposalLayer& L = spk::kProposalSpec[l];
-            s = spk::alloc(net, net->w[l], static_cast<std::size_t>(L.cout) * 27 * spk::cin_pad(L.cin));
+            s = spk::alloc(ctx, net, net->w[l], static_cast<std::size_t>(L.cout) * 27 * spk::cin_pad(L.cin));
         }
         if (s) {
             for (void* q : net->owned) {
@@ -1983,7 +1982,7 @@ int spk_proposal_forward(spk_context* ctx, spk_proposal* p, uint64_t batch, cons
             return spk::kInvalidArgument;
         }
         const auto b = static_cast<std::uint32_t>(batch);
-        int s = spk::ensure_batch(net, b);
+        int s = spk::ensure_batch(ctx, net, b);
         if (!s) s = spk::upload_inputs(ctx, net, b, inputs);
         if (!s) s = spk::launch_forward(ctx, net, b);
         if (s) {
@@ -2014,7 +2013,7 @@ int spk_proposal_gradients(spk_context* ctx, spk_proposal* p, uint64_t batch, co
             return spk::kInvalidArgument;
         }
         const auto b = static_cast<std::uint32_t>(batch);
-        int s = spk::ensure_batch(net, b);
+        int s = spk::ensure_batch(ctx, net, b);
         if (!s) s = spk::upload_inputs(ctx, net, b, inputs);
         if (s) {
             return s;
@@ -2046,7 +2045,7 @@ int spk_proposal_train(spk_context* ctx, spk_proposal* p, const spk_proposal_dat
                 return spk::kInvalidArgument;
             }
         }
-        int s = spk::ensure_batch(net, batch);
+        int s = spk::ensure_batch(ctx, net, batch);
         if (s) {
             return s;
         }

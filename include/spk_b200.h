@@ -89,7 +89,9 @@ typedef struct spk_control {
 /* Opens a context on `device` with a device-memory cap (0 = no cap).  It
  * holds what the reference's FftExecution holds (make_fft_execution,
  * correlation.hpp:80-98): execution resources reused across calls, which one
- * coordinator serialises (correlation.hpp:78-79). */
+ * coordinator serialises (correlation.hpp:78-79).  The cap is on the calls'
+ * fields and working buffers; an open session's kernel spectra and a proposal
+ * network's data lie outside it. */
 int spk_context_create(int device, uint64_t max_device_bytes, spk_context** out);
 void spk_context_destroy(spk_context* context);
 /* Static string for a status (e.g. "CORRELATION_NUMERIC"); never NULL.  The
