@@ -46,14 +46,16 @@ struct Shared {
     std::condition_variable posted, left;
     std::vector<Work*> work;
     std::vector<std::thread> helpers;
-    bool stop {};
+    // Helpers end when their generation is over.  The last context to go ends
+    // it; contexts opened while it still joins them get helpers of the next.
+    unsigned generation {};
 
-    void serve()
+    void serve(unsigned mine)
     {
         std::unique_lock<std::mutex> hold(lock);
         for (;;) {
-            posted.wait(hold, [&] { return stop || !work.empty(); });
-            if (stop) {
+            posted.wait(hold, [&] { return generation != mine || !work.empty(); });
+            if (generation != mine) {
                 return;
             }
             Work* w = work.back();
@@ -163,7 +165,7 @@ public:
             const std::lock_guard<std::mutex> hold(p.lock);
             try {
                 while (p.helpers.size() < want) {
-                    p.helpers.emplace_back([&p] { p.serve(); });
+                    p.helpers.emplace_back([&p, mine = p.generation] { p.serve(mine); });
                 }
                 work_.tickets = want;
                 p.work.insert(p.work.begin(), &work_);
@@ -230,14 +232,12 @@ void copy_resources_release()
         p.chunks.clear();
         p.free.clear();
         helpers.swap(p.helpers);
-        p.stop = true;
+        ++p.generation;
     }
     p.posted.notify_all();
     for (auto& t : helpers) {
         t.join();
     }
-    const std::lock_guard<std::mutex> hold(p.lock);
-    p.stop = false;
 }
 
 int copy_to_host(spk_context* ctx, void* dst, const void* d_src, std::size_t bytes)
