@@ -254,16 +254,24 @@ int copy_to_host(spk_context* ctx, void* dst, const void* d_src, std::size_t byt
             std::memcpy(static_cast<char*>(dst) + i * kSlotBytes, slots.slot[i % c.slots], c.size(i));
             c.finished[i].store(true, std::memory_order_release);
         };
+        // After a failure nothing is in flight any more, and every chunk counts as
+        // arrived, so that nobody waits.
+        const auto broken = [&] {
+            ok = false;
+            cudaStreamSynchronize(st);
+        };
         // This thread keeps the slots filling and sees them arrive; the helpers
         // empty them without calling CUDA.
         std::size_t issued = 0;
         const auto issue = [&] {
             while (issued < c.count &&
                    (issued < c.slots || c.finished[issued - c.slots].load(std::memory_order_acquire))) {
-                ok = ok &&
-                     cudaMemcpyAsync(slots.slot[issued % c.slots], static_cast<const char*>(d_src) + issued * kSlotBytes,
-                                     c.size(issued), cudaMemcpyDeviceToHost, st) == cudaSuccess &&
-                     cudaEventRecord(ctx->copy_events[issued % c.slots], st) == cudaSuccess;
+                if (ok &&
+                    (cudaMemcpyAsync(slots.slot[issued % c.slots], static_cast<const char*>(d_src) + issued * kSlotBytes,
+                                     c.size(issued), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                     cudaEventRecord(ctx->copy_events[issued % c.slots], st) != cudaSuccess)) {
+                    broken();
+                }
                 ++issued;
             }
         };
@@ -280,14 +288,17 @@ int copy_to_host(spk_context* ctx, void* dst, const void* d_src, std::size_t byt
         };
         // Woken while the work before the copy runs.
         const Helpers helpers(bytes, help);
-        ok = ok && cudaEventSynchronize(ctx->copy_events[0]) == cudaSuccess;
+        if (ok && cudaEventSynchronize(ctx->copy_events[0]) != cudaSuccess) {
+            broken();
+        }
         std::size_t arrived = 0;
         while (arrived < c.count) {
             issue();
             const cudaError_t state = ok ? cudaEventQuery(ctx->copy_events[arrived % c.slots]) : cudaErrorUnknown;
             if (arrived < issued && state != cudaErrorNotReady) {
-                // After a failure every chunk counts as arrived, so that nobody waits.
-                ok = ok && state == cudaSuccess;
+                if (ok && state != cudaSuccess) {
+                    broken();
+                }
                 c.arrived.store(++arrived, std::memory_order_release);
                 continue;
             }
@@ -333,20 +344,29 @@ int copy_to_device(spk_context* ctx, void* d_dst, const void* src, std::size_t b
                     fill(i);
                 }
             });
+            // As in copy_to_host: the slots go back with nothing in flight.
+            const auto broken = [&] {
+                ok = false;
+                cudaStreamSynchronize(st);
+            };
             std::size_t issued = 0, arrived = 0;
             while (arrived < c.count) {
                 if (issued < c.count && c.finished[issued].load(std::memory_order_acquire)) {
-                    ok = ok &&
-                         cudaMemcpyAsync(static_cast<char*>(d_dst) + issued * kSlotBytes, slots.slot[issued % c.slots],
-                                         c.size(issued), cudaMemcpyHostToDevice, st) == cudaSuccess &&
-                         cudaEventRecord(ctx->copy_events[issued % c.slots], st) == cudaSuccess;
+                    if (ok &&
+                        (cudaMemcpyAsync(static_cast<char*>(d_dst) + issued * kSlotBytes, slots.slot[issued % c.slots],
+                                         c.size(issued), cudaMemcpyHostToDevice, st) != cudaSuccess ||
+                         cudaEventRecord(ctx->copy_events[issued % c.slots], st) != cudaSuccess)) {
+                        broken();
+                    }
                     ++issued;
                     continue;
                 }
                 if (arrived < issued) {
                     const cudaError_t state = ok ? cudaEventQuery(ctx->copy_events[arrived % c.slots]) : cudaErrorUnknown;
                     if (state != cudaErrorNotReady) {
-                        ok = ok && state == cudaSuccess;
+                        if (ok && state != cudaSuccess) {
+                            broken();
+                        }
                         c.arrived.store(++arrived, std::memory_order_release);
                         continue;
                     }

@@ -276,6 +276,37 @@ void helpers_live()
           "every helper is at work after contexts came and went");
 }
 
+// A copy that fails keeps its slots until its DMAs are over.
+void failing_copy()
+{
+    const std::size_t n = 40 * MB;
+    const auto source = pattern(n, 5);
+    std::vector<char> device(n);
+    for (int after : { 0, 1, 5, 17, 40 }) {
+        Context c;
+        { Context warm; round_trip(warm, n, 1); }
+        bool early = false;
+        on_synchronize = [&] {
+            const std::lock_guard<std::mutex> hold(spk::shared().lock);
+            early = early || (!c.stream.queue.empty() &&
+                              spk::shared().free.size() == spk::shared().chunks.size() * spk::kChunkSlots);
+        };
+        fail_copy_after = after;
+        const int to_device = spk::copy_to_device(&c.ctx, device.data(), source.data(), n);
+        const bool drained = c.stream.queue.empty();
+        fail_copy_after = -1;
+        on_synchronize = nullptr;
+        check(to_device == spk::kCuda, "a failing copy to the device says so");
+        check(drained, "and leaves nothing in flight");
+        check(!early, "and holds its slots until then");
+        fail_copy_after = after;
+        const int to_host = spk::copy_to_host(&c.ctx, device.data(), source.data(), n);
+        fail_copy_after = -1;
+        check(to_host == spk::kCuda && c.stream.queue.empty(), "a failing copy to the host likewise");
+        check(round_trip(c, n, 9), "the next copy is whole");
+    }
+}
+
 }  // namespace
 
 int main(int, char** argv)
@@ -292,6 +323,9 @@ int main(int, char** argv)
     }
     else if (which == "helpers_live") {
         helpers_live();
+    }
+    else if (which == "failing_copy") {
+        failing_copy();
     }
     else {
         return 2;
