@@ -1,10 +1,13 @@
 #include "host_copy.hpp"
 
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
 #include <condition_variable>
+#include <cstdint>
 #include <cstring>
 #include <functional>
 #include <memory>
@@ -22,9 +25,31 @@ constexpr std::size_t kSlotBytes = 512 << 10;
 constexpr std::size_t kMaxThreads = 4;
 constexpr std::size_t kChunkSlots = 8;  // slots pinned at once
 constexpr std::size_t kMaxSlots = 16;
-// Copies from this size on wake helpers: it costs up to 200 us where the cores
-// idle (a 4 MB copy took 0.85 ms with one and 0.59 without).
+// Which way is the fastest depends on the size and on what the CPU last did
+// with the destination's pages: medians in us, 200 to 300 us apart, so that
+// helpers sleep in between and cost up to 300 us to wake.
+//
+//   MB to the host               0.5    1  1.5    2    4    8   10   16    33
+//   touched, not lately  plain    50   84  116  139  249  484  576  866  1634
+//                        slots    54   88  122  156  300  669  884 1681  2177
+//                        helped                      511  614  651  587   980
+//   just written         plain    82  133  180  218  302  576  831 1076
+//                        slots    44   69  107  147  298  638  870 1555
+//   never touched        plain   250  471       920 1828 3578 4543 7262 14934
+//                        slots   152  282       557 1097 2159 2798 4454 11570
+//                        helped                      981 1290 1253 1500  2897
+//   to the device        plain    40   68       112  229  432  540  840  1728
+//                        slots    44   73       154  285  541  683 1073  2201
+//                        helped                      367  699  830 1237  1701
+//
+// The driver's own way faults untouched pages in as it goes: slots win at any
+// size there, with helpers from 4 to 8 MB on.  Into touched pages slots cost at
+// most 5 us more up to 1.5 MB and save up to 70; beyond, up to 40% more, until
+// helpers pay at about 12 MB.  Sources take the plain way up to 32 MB.
+constexpr std::size_t kSmallBytes = 3 << 19;
 constexpr std::size_t kHelpedBytes = 8 << 20;
+constexpr std::size_t kTouchedBytes = 12 << 20;
+constexpr std::size_t kSourceBytes = 32 << 20;
 // Bytes that pay for a helper more.
 constexpr std::size_t kBytesPerThread = 3 << 20;
 
@@ -149,14 +174,35 @@ void wait_until(const Condition& condition)
     }
 }
 
+// Whether more than a sixteenth of `bytes` < kTouchedBytes from `at` on lies in
+// pages that were never touched: from there on the slots' 10 us per MB more are
+// less than the 180 us per MB that they save on those pages.
+bool untouched(const void* at, std::size_t bytes)
+{
+    const auto page = static_cast<std::uintptr_t>(sysconf(_SC_PAGESIZE));
+    const std::uintptr_t first = reinterpret_cast<std::uintptr_t>(at) / page * page;
+    const std::size_t pages = (reinterpret_cast<std::uintptr_t>(at) + bytes - first + page - 1) / page;
+    unsigned char resident[kTouchedBytes / 4096 + 2];
+    if (pages > sizeof(resident) || mincore(reinterpret_cast<void*>(first), pages * page, resident) != 0) {
+        return false;
+    }
+    const auto missing =
+        static_cast<std::size_t>(std::count_if(resident, resident + pages, [](unsigned char r) { return !(r & 1); }));
+    return missing > pages / 16;
+}
+
+std::size_t most_helpers()
+{
+    return std::min<std::size_t>(kMaxThreads, std::thread::hardware_concurrency() / 2);
+}
+
 // Helper threads at work on a copy until the end of the scope.  There may be
 // fewer than wanted, or none: the calling thread takes any chunk no helper has.
 class Helpers {
 public:
     Helpers(std::size_t bytes, std::function<void()> body) : work_ { std::move(body), 0, 0 }
     {
-        const std::size_t cores = std::max(1U, std::thread::hardware_concurrency());
-        const std::size_t want = std::min({ kMaxThreads, cores / 2, bytes / kBytesPerThread });
+        const std::size_t want = std::min(most_helpers(), bytes / kBytesPerThread);
         if (bytes < kHelpedBytes || !want) {
             return;
         }
@@ -244,7 +290,8 @@ int copy_to_host(spk_context* ctx, void* dst, const void* d_src, std::size_t byt
 {
     cudaStream_t st = ctx->stream;
     bool ok = true;
-    Slots slots(ctx, std::min((bytes + kSlotBytes - 1) / kSlotBytes, kMaxSlots));
+    const bool staged = bytes <= kSmallBytes || (bytes < kTouchedBytes ? untouched(dst, bytes) : most_helpers() > 1);
+    Slots slots(ctx, staged ? std::min((bytes + kSlotBytes - 1) / kSlotBytes, kMaxSlots) : 0);
     if (!slots.usable()) {
         ok = !bytes || cudaMemcpyAsync(dst, d_src, bytes, cudaMemcpyDeviceToHost, st) == cudaSuccess;
     }
@@ -320,7 +367,7 @@ int copy_to_device(spk_context* ctx, void* d_dst, const void* src, std::size_t b
 {
     cudaStream_t st = ctx->stream;
     bool ok = true;
-    if (bytes < (4 << 20)) {  // the driver copies a small source at once
+    if (bytes < kSourceBytes || most_helpers() < 2) {
         ok = cudaMemcpyAsync(d_dst, src, bytes, cudaMemcpyHostToDevice, st) == cudaSuccess;
     }
     else {

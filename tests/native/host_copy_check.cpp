@@ -57,6 +57,7 @@ int fail_copy_after = -1;  // that many copies succeed
 std::atomic<long long> pinned { 0 };
 std::atomic<int> pin_calls { 0 };
 bool pin_fails = false;
+std::size_t largest_dma = 0;
 std::function<void()> on_synchronize;
 
 int failures = 0;
@@ -91,6 +92,7 @@ cudaError_t cudaMemcpyAsync(void* to, const void* from, size_t bytes, cudaMemcpy
         return cudaErrorUnknown;
     }
     fail_copy_after -= fail_copy_after > 0;
+    largest_dma = std::max(largest_dma, bytes);
     fake(s)->queue.push_back({ to, from, bytes, nullptr });
     return cudaSuccess;
 }
@@ -209,10 +211,44 @@ void sizes()
 {
     Context c;
     for (std::size_t n : { std::size_t { 1 }, 4 * KB, 512 * KB - 1, 512 * KB, 512 * KB + 1, 1 * MB, 4 * MB - 1, 4 * MB,
-                           4 * MB + 1, 8 * MB - 1, 8 * MB, 8 * MB + 1, 9 * MB + 7, 33 * MB, 33 * MB + 5 }) {
+                           4 * MB + 1, 8 * MB - 1, 8 * MB, 8 * MB + 1, 12 * MB - 1, 12 * MB + 1, 33 * MB, 33 * MB + 5 }) {
         check(round_trip(c, n, static_cast<unsigned>(n)), "a copy's bytes");
     }
     check(spk::copy_to_host(&c.ctx, nullptr, nullptr, 0) == spk::kOk, "no bytes");
+}
+
+// Which copies go through slots: DMAs of a slot at most.
+void ways()
+{
+    Context c;
+    const bool helped = spk::most_helpers() > 1;
+    const auto staged = [&](std::size_t n, bool to_device, bool touched) {
+        char* host = static_cast<char*>(mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0));
+        if (touched) {
+            std::memset(host, 1, n);
+        }
+        std::vector<char> device(n, 2);
+        largest_dma = 0;
+        const int status = to_device ? spk::copy_to_device(&c.ctx, device.data(), host, n)
+                                     : spk::copy_to_host(&c.ctx, host, device.data(), n);
+        cudaStreamSynchronize(c.ctx.stream);
+        check(status == spk::kOk && std::memcmp(host, device.data(), n) == 0, "a copy's bytes");
+        munmap(host, n);
+        return largest_dma < n;
+    };
+    for (std::size_t n : { 4 * KB, 512 * KB, 3 * MB / 2 }) {
+        check(staged(n, false, true) == (n > 512 * KB) && staged(n, false, false) == (n > 512 * KB),
+              "small copies take the slots, in one piece up to a slot");
+    }
+    for (std::size_t mb : { 2, 3, 7, 8, 11 }) {
+        check(!staged(mb * MB, false, true), "touched pages below 12 MB take the plain way");
+        check(staged(mb * MB, false, false), "untouched pages take the slots");
+        check(!staged(mb * MB, true, true), "sources below 32 MB take the plain way");
+    }
+    for (std::size_t mb : { 12, 16, 31, 32, 50 }) {
+        check(staged(mb * MB, false, true) == helped, "larger copies take the slots where there are helpers");
+        check(staged(mb * MB, true, true) == (helped && mb >= 32), "and larger sources");
+    }
 }
 
 void no_slots()
@@ -314,6 +350,9 @@ int main(int, char** argv)
     const std::string which = argv[1];
     if (which == "sizes") {
         sizes();
+    }
+    else if (which == "ways") {
+        ways();
     }
     else if (which == "no_slots") {
         no_slots();
