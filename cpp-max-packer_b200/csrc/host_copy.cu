@@ -50,6 +50,14 @@ constexpr std::size_t kSmallBytes = 3 << 19;
 constexpr std::size_t kHelpedBytes = 8 << 20;
 constexpr std::size_t kTouchedBytes = 12 << 20;
 constexpr std::size_t kSourceBytes = 32 << 20;
+double mega(std::size_t bytes) { return static_cast<double>(bytes) / (1 << 20); }
+
+// Pinning a chunk of slots and giving it back costs 2.5 to 8 ms, which a context
+// that makes a few small copies never gets back.  Copies therefore take the
+// plain way until what slots would have saved them (us per MB, from the table)
+// comes to that.
+constexpr double kPinCost = 3000;
+constexpr double kSavedUntouched = 180, kSavedTouched = 30;
 // Bytes that pay for a helper more.
 constexpr std::size_t kBytesPerThread = 3 << 20;
 
@@ -61,6 +69,7 @@ struct Shared {
     int contexts {};
     std::vector<char*> free;     // slots nobody has checked out
     std::vector<void*> chunks;   // their allocations
+    double earned {};            // us that slots have saved, or would have
 
     // Helpers wait for posted work.  A ticket is one helper's share of a copy.
     struct Work {
@@ -106,16 +115,18 @@ Shared& shared()
     return *s;
 }
 
-// Up to `want` slots checked out for one copy, with the context's events beside
-// them; returned when the copy is done with them.
+// Up to `want` slots checked out for one copy, which saves `saved` us by them,
+// with the context's events beside them; returned when the copy is done with them.
 class Slots {
 public:
-    Slots(spk_context* ctx, std::size_t want)
+    Slots(spk_context* ctx, std::size_t want, double saved)
     {
         Shared& p = shared();
         {
             const std::lock_guard<std::mutex> hold(p.lock);
-            while (p.free.size() < want && p.chunks.size() * kChunkSlots < kMaxSlots) {
+            p.earned += saved;
+            while (p.free.size() < want && p.chunks.size() * kChunkSlots < kMaxSlots &&
+                   p.earned >= kPinCost * static_cast<double>(p.chunks.size() + 1)) {
                 void* chunk {};
                 if (cudaHostAlloc(&chunk, kChunkSlots * kSlotBytes, cudaHostAllocPortable) != cudaSuccess) {
                     cudaGetLastError();
@@ -174,21 +185,24 @@ void wait_until(const Condition& condition)
     }
 }
 
-// Whether more than a sixteenth of `bytes` < kTouchedBytes from `at` on lies in
-// pages that were never touched: from there on the slots' 10 us per MB more are
-// less than the 180 us per MB that they save on those pages.
+// Whether more than a sixteenth of `bytes` from `at` on lies in pages that were
+// never touched, as far as both ends tell: from there on the slots' 10 us per MB
+// more are less than the 180 us per MB that they save on those pages.
 bool untouched(const void* at, std::size_t bytes)
 {
+    constexpr std::size_t most = 256;  // pages asked about at each end
     const auto page = static_cast<std::uintptr_t>(sysconf(_SC_PAGESIZE));
-    const std::uintptr_t first = reinterpret_cast<std::uintptr_t>(at) / page * page;
-    const std::size_t pages = (reinterpret_cast<std::uintptr_t>(at) + bytes - first + page - 1) / page;
-    unsigned char resident[kTouchedBytes / 4096 + 2];
-    if (pages > sizeof(resident) || mincore(reinterpret_cast<void*>(first), pages * page, resident) != 0) {
+    const std::uintptr_t first = reinterpret_cast<std::uintptr_t>(at) / page;
+    const std::size_t pages = (reinterpret_cast<std::uintptr_t>(at) + bytes + page - 1) / page - first;
+    const std::size_t head = std::min(pages, most), tail = std::min(pages - head, most);
+    unsigned char resident[2 * most];
+    if (!bytes || mincore(reinterpret_cast<void*>(first * page), head * page, resident) != 0 ||
+        (tail && mincore(reinterpret_cast<void*>((first + pages - tail) * page), tail * page, resident + head) != 0)) {
         return false;
     }
-    const auto missing =
-        static_cast<std::size_t>(std::count_if(resident, resident + pages, [](unsigned char r) { return !(r & 1); }));
-    return missing > pages / 16;
+    const auto missing = static_cast<std::size_t>(
+        std::count_if(resident, resident + head + tail, [](unsigned char r) { return !(r & 1); }));
+    return missing > (head + tail) / 16;
 }
 
 std::size_t most_helpers()
@@ -277,6 +291,7 @@ void copy_resources_release()
         }
         p.chunks.clear();
         p.free.clear();
+        p.earned = 0;
         helpers.swap(p.helpers);
         ++p.generation;
     }
@@ -290,8 +305,10 @@ int copy_to_host(spk_context* ctx, void* dst, const void* d_src, std::size_t byt
 {
     cudaStream_t st = ctx->stream;
     bool ok = true;
-    const bool staged = bytes <= kSmallBytes || (bytes < kTouchedBytes ? untouched(dst, bytes) : most_helpers() > 1);
-    Slots slots(ctx, staged ? std::min((bytes + kSlotBytes - 1) / kSlotBytes, kMaxSlots) : 0);
+    const bool fresh = untouched(dst, bytes);
+    const bool staged = fresh || bytes <= kSmallBytes || (bytes >= kTouchedBytes && most_helpers() > 1);
+    Slots slots(ctx, staged ? std::min((bytes + kSlotBytes - 1) / kSlotBytes, kMaxSlots) : 0,
+                staged ? mega(bytes) * (fresh ? kSavedUntouched : kSavedTouched) : 0.0);
     if (!slots.usable()) {
         ok = !bytes || cudaMemcpyAsync(dst, d_src, bytes, cudaMemcpyDeviceToHost, st) == cudaSuccess;
     }
@@ -371,7 +388,7 @@ int copy_to_device(spk_context* ctx, void* d_dst, const void* src, std::size_t b
         ok = cudaMemcpyAsync(d_dst, src, bytes, cudaMemcpyHostToDevice, st) == cudaSuccess;
     }
     else {
-        Slots slots(ctx, kMaxSlots);
+        Slots slots(ctx, kMaxSlots, mega(bytes) * kSavedTouched);
         if (!slots.usable()) {
             ok = cudaMemcpyAsync(d_dst, src, bytes, cudaMemcpyHostToDevice, st) == cudaSuccess;
         }

@@ -221,6 +221,7 @@ void sizes()
 void ways()
 {
     Context c;
+    check(round_trip(c, 64 * MB, 1), "a copy that earns both chunks of slots");
     const bool helped = spk::most_helpers() > 1;
     const auto staged = [&](std::size_t n, bool to_device, bool touched) {
         char* host = static_cast<char*>(mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0));
@@ -249,6 +250,43 @@ void ways()
         check(staged(mb * MB, false, true) == helped, "larger copies take the slots where there are helpers");
         check(staged(mb * MB, true, true) == (helped && mb >= 32), "and larger sources");
     }
+}
+
+// Slots are pinned once copies have earned them, and go with the last context.
+void pins()
+{
+    std::vector<char> device(80 * MB, 1);
+    const auto untouched_copy = [&](Context& c, std::size_t n) {
+        char* to = static_cast<char*>(mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0));
+        check(spk::copy_to_host(&c.ctx, to, device.data(), n) == spk::kOk && std::memcmp(to, device.data(), n) == 0,
+              "a copy's bytes");
+        munmap(to, n);
+    };
+    for (int i = 0; i < 40; ++i) {
+        Context c;
+        untouched_copy(c, 2 * MB);
+        untouched_copy(c, 400 * KB);
+    }
+    check(pin_calls == 0, "contexts that make a few small copies pin nothing");
+    {
+        Context c;
+        for (int i = 0; i < 20; ++i) {
+            untouched_copy(c, 2 * MB);
+        }
+        check(pin_calls == 1 && pinned == static_cast<long long>(4 * MB), "many small copies pin one chunk");
+        for (int i = 0; i < 20; ++i) {
+            untouched_copy(c, 20 * MB);
+        }
+        check(pin_calls == 2 && pinned == static_cast<long long>(8 * MB), "large ones two, and no more");
+    }
+    check(pinned == 0, "the last context gives them back");
+    pin_calls = 0;
+    {
+        Context c;
+        untouched_copy(c, 80 * MB);
+        check(pin_calls == 2, "one large copy earns both at once");
+    }
+    check(pinned == 0, "and gives them back");
 }
 
 void no_slots()
@@ -353,6 +391,9 @@ int main(int, char** argv)
     }
     else if (which == "ways") {
         ways();
+    }
+    else if (which == "pins") {
+        pins();
     }
     else if (which == "no_slots") {
         no_slots();
