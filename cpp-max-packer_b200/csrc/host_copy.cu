@@ -27,12 +27,13 @@ constexpr std::size_t kChunkSlots = 8;  // slots pinned at once
 constexpr std::size_t kMaxSlots = 16;
 // Which way is the fastest depends on the size and on what the CPU last did
 // with the destination's pages: medians in us, 200 to 300 us apart, so that
-// helpers sleep in between and cost up to 300 us to wake.
+// helpers sleep in between and cost up to 300 us to wake (two boxes).
 //
 //   MB to the host               0.5    1  1.5    2    4    8   10   16    33
 //   touched, not lately  plain    50   84  116  139  249  484  576  866  1634
 //                        slots    54   88  122  156  300  669  884 1681  2177
-//                        helped                      511  614  651  587   980
+//                        helped                 208  401  405  660   980
+//                                               511  614  651  587
 //   just written         plain    82  133  180  218  302  576  831 1076
 //                        slots    44   69  107  147  298  638  870 1555
 //   never touched        plain   250  471       920 1828 3578 4543 7262 14934
@@ -45,11 +46,16 @@ constexpr std::size_t kMaxSlots = 16;
 // The driver's own way faults untouched pages in as it goes: slots win at any
 // size there, with helpers from 4 to 8 MB on.  Into touched pages slots cost at
 // most 5 us more up to 1.5 MB and save up to 70; beyond, up to 40% more, until
-// helpers pay at about 12 MB.  Sources take the plain way up to 32 MB.
+// helpers pay: at 3 MB where they wake fast, at 12 where they do not, so from 8
+// on (a program that asks for 11 MB proximity fields: 0.83 ms a call the plain
+// way, 0.52 this way).  The sources above were read shortly before.  From memory,
+// inputs of FP32 correlations, whole calls in ms with plain copies, slots from 4
+// and helped slots from 8 MB: 4.2 MB 0.85, 1.08, 0.9; 6.5 MB 1.06, 1.45, 1.3; 9 MB
+// 1.4, 1.58, 1.57; 12 MB 1.82, 1.74, 1.72; 15 MB 2.38, 2.06, 2.11; 26 MB 3.82, 3.08,
+// 2.92: plain below 12 MB.
 constexpr std::size_t kSmallBytes = 3 << 19;
 constexpr std::size_t kHelpedBytes = 8 << 20;
-constexpr std::size_t kTouchedBytes = 12 << 20;
-constexpr std::size_t kSourceBytes = 32 << 20;
+constexpr std::size_t kSourceBytes = 12 << 20;
 double mega(std::size_t bytes) { return static_cast<double>(bytes) / (1 << 20); }
 
 // Pinning a chunk of slots and giving it back costs 2.5 to 8 ms, which a context
@@ -306,7 +312,7 @@ int copy_to_host(spk_context* ctx, void* dst, const void* d_src, std::size_t byt
     cudaStream_t st = ctx->stream;
     bool ok = true;
     const bool fresh = untouched(dst, bytes);
-    const bool staged = fresh || bytes <= kSmallBytes || (bytes >= kTouchedBytes && most_helpers() > 1);
+    const bool staged = fresh || bytes <= kSmallBytes || (bytes >= kHelpedBytes && most_helpers() > 1);
     Slots slots(ctx, staged ? std::min((bytes + kSlotBytes - 1) / kSlotBytes, kMaxSlots) : 0,
                 staged ? mega(bytes) * (fresh ? kSavedUntouched : kSavedTouched) : 0.0);
     if (!slots.usable()) {

@@ -211,7 +211,7 @@ void sizes()
 {
     Context c;
     for (std::size_t n : { std::size_t { 1 }, 4 * KB, 512 * KB - 1, 512 * KB, 512 * KB + 1, 1 * MB, 4 * MB - 1, 4 * MB,
-                           4 * MB + 1, 8 * MB - 1, 8 * MB, 8 * MB + 1, 12 * MB - 1, 12 * MB + 1, 33 * MB, 33 * MB + 5 }) {
+                           4 * MB + 1, 8 * MB - 1, 8 * MB, 8 * MB + 1, 12 * MB + 1, 33 * MB, 33 * MB + 5 }) {
         check(round_trip(c, n, static_cast<unsigned>(n)), "a copy's bytes");
     }
     check(spk::copy_to_host(&c.ctx, nullptr, nullptr, 0) == spk::kOk, "no bytes");
@@ -241,14 +241,14 @@ void ways()
         check(staged(n, false, true) == (n > 512 * KB) && staged(n, false, false) == (n > 512 * KB),
               "small copies take the slots, in one piece up to a slot");
     }
-    for (std::size_t mb : { 2, 3, 7, 8, 11 }) {
-        check(!staged(mb * MB, false, true), "touched pages below 12 MB take the plain way");
+    for (std::size_t mb : { 2, 3, 5, 7 }) {
+        check(!staged(mb * MB, false, true), "touched pages below 8 MB take the plain way");
         check(staged(mb * MB, false, false), "untouched pages take the slots");
-        check(!staged(mb * MB, true, true), "sources below 32 MB take the plain way");
+        check(!staged(mb * MB, true, true), "sources below 12 MB take the plain way");
     }
-    for (std::size_t mb : { 12, 16, 31, 32, 50 }) {
+    for (std::size_t mb : { 8, 11, 12, 16, 50 }) {
         check(staged(mb * MB, false, true) == helped, "larger copies take the slots where there are helpers");
-        check(staged(mb * MB, true, true) == (helped && mb >= 32), "and larger sources");
+        check(staged(mb * MB, true, true) == (helped && mb >= 12), "and larger sources");
     }
 }
 
