@@ -286,7 +286,7 @@ def correlate_binary_mask(spec: CorrelationSpec, environment, kernel, box_first:
     bf = (ctypes.c_int64 * 3)(*[int(v) for v in box_first])
     bs = (ctypes.c_uint32 * 3)(*[int(v) for v in box_shape])
     count = int(np.prod([int(v) for v in box_shape], dtype=np.int64))
-    mask = np.zeros(max(count, 1), np.uint8)
+    mask = np.empty(max(count, 1), np.uint8)
     cap = count if capacity is None else int(capacity)
     res = _lib.CorrelationResultC()
     lim = _lib.CorrelationLimits(limits.max_working_bytes, limits.reserved_bytes, limits.max_padded_cells,

@@ -95,7 +95,7 @@ def voxelize_container(container: Union[Sequence[float], AcceptedMesh], origin_m
     lib = _lib_ready()
     context = context or default_context()
     f, s = _arr(first, np.int64), _arr(shape, np.uint32)
-    cells = np.zeros(int(np.prod(s.astype(np.int64))), np.uint8)
+    cells = np.empty(int(np.prod(s.astype(np.int64))), np.uint8)
     o = _arr(origin_mm, np.float64)
     if isinstance(container, AcceptedMesh):
         mc, keep = _mesh_c(container)
@@ -115,7 +115,7 @@ def voxelize_placed(mesh: AcceptedMesh, origin_mm, pitch_mm, first, shape, trans
     context = context or default_context()
     mc, keep = _mesh_c(mesh)
     f, s = _arr(first, np.int64), _arr(shape, np.uint32)
-    cells = np.zeros(int(np.prod(s.astype(np.int64))), np.uint8)
+    cells = np.empty(int(np.prod(s.astype(np.int64))), np.uint8)
     o, t, q = _arr(origin_mm, np.float64), _arr(translation_mm, np.float64), _arr(q_xyzw, np.float64)
     status = lib.spk_voxelize_placed(context.handle, ctypes.byref(mc), o.ctypes.data, pitch_mm, f.ctypes.data,
                                      s.ctypes.data, t.ctypes.data, q.ctypes.data, pair_clearance_mm,

@@ -207,7 +207,7 @@ class Session:
         _lib.check(self.lib.spk_session_field(self.context.handle, code, orientation, first.ctypes.data,
                                               shape.ctypes.data, None, 0), "spk_session_field")
         n = int(np.prod(shape.astype(np.int64)))
-        out = np.zeros(n, np.float64 if code == 3 else np.uint8)
+        out = np.empty(n, np.float64 if code == 3 else np.uint8)
         _lib.check(self.lib.spk_session_field(self.context.handle, code, orientation, first.ctypes.data,
                                               shape.ctypes.data, out.ctypes.data, out.nbytes), "spk_session_field")
         self.last_window = (tuple(int(v) for v in first), tuple(int(v) for v in shape))
