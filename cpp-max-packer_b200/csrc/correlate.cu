@@ -587,6 +587,12 @@ int correlate(spk_context* ctx, const spk_correlation_spec* spec_ptr, const E* e
     std::uint8_t* d_ker = d_in + ker_at;
     auto* d_out = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(d_back) + out_at);
     cudaStream_t st = ctx->stream;
+    // A call that stops early waits for what it has launched: the pinned
+    // copies of its inputs are the context's.
+    const auto stop = [&](int s) {
+        cudaStreamSynchronize(st);
+        return s;
+    };
     if (small_in) {
         std::memcpy(in, environment, env_count * sizeof(E));
         std::memcpy(in + ker_at, kernel, ker_count);
@@ -594,7 +600,7 @@ int correlate(spk_context* ctx, const spk_correlation_spec* spec_ptr, const E* e
     }
     else if ((status = copy_to_device(ctx, d_env, environment, env_count * sizeof(E))) ||
              (status = copy_to_device(ctx, d_ker, kernel, ker_count))) {
-        return status;
+        return stop(status);
     }
     cudaMemsetAsync(d_back, 0, sizeof(Readback), st);
     validate_kernel<E><<<validate_blocks, kValidateThreads, 0, st>>>(
@@ -605,24 +611,18 @@ int correlate(spk_context* ctx, const spk_correlation_spec* spec_ptr, const E* e
     // FP64 keeps the reference's 1e-10 proximity tolerance; FP32 states its
     // own bound, 2^-13 relative to the output scale (2^-8 with FP16 spectra).
     const double rel = sizeof(T) == 8 ? 1e-10 : half_spectra ? 1.0 / 256.0 : 1.0 / 8192.0;
-    // A call that stops early waits for what it has launched: the pinned
-    // copies of its inputs are the context's.
-    const auto stop = [&](int s) {
-        cudaStreamSynchronize(st);
-        return s;
-    };
     if constexpr (staged) {
         for (int a = 0; a != 3; ++a) {
             stages.roots[a] = twiddle_table<T>(ctx, L[a], status);
             if (!stages.roots[a]) {
-                return status;
+                return stop(status);
             }
         }
         stages.z = z;
         stages.w = w;
         stages.stream = st;
         if ((status = stages.forward(d_env, d_ker))) {
-            return status;
+            return stop(status);
         }
         if (int s = poll(control)) {
             return stop(s);
@@ -635,19 +635,19 @@ int correlate(spk_context* ctx, const spk_correlation_spec* spec_ptr, const E* e
             cudaMemcpyAsync(&back->input, &d_back->input, sizeof(InputStats), cudaMemcpyDeviceToHost, st);
             if (cudaStreamSynchronize(st) != cudaSuccess) {
                 cudaGetLastError();
-                return kCuda;
+                return stop(kCuda);
             }
             const double bound = (binary ? static_cast<double>(back->input.env_ones) : back->input.mass) +
                                  static_cast<double>(back->input.ker_ones);
             shift = bound > 0 ? 15 - static_cast<int>(std::ceil(std::log2(bound))) : 0;
             zh = static_cast<__half2*>(device_buffer(ctx, "corr.zh", half_bytes, status));
             if (!zh || (status = stages.to_half(zh, shift))) {
-                return status;
+                return stop(status);
             }
             ctx->launches++;
         }
         if ((status = stages.back(zh, shift, &d_back->input, binary, rel, d_out, d_stats, &d_back->flags))) {
-            return status;
+            return stop(status);
         }
         if (int s = poll(control)) {
             return stop(s);
@@ -658,25 +658,25 @@ int correlate(spk_context* ctx, const spk_correlation_spec* spec_ptr, const E* e
         for (int a = 0; a != 3; ++a) {
             passes.roots[a] = twiddle_table<T>(ctx, L[a], status);
             if (!passes.roots[a]) {
-                return status;
+                return stop(status);
             }
         }
         passes.z = z;
         passes.stream = st;
         if ((status = passes.forward(d_env, d_ker))) {
-            return status;
+            return stop(status);
         }
         if (int s = poll(control)) {
             return stop(s);
         }
         if ((status = passes.multiply())) {
-            return status;
+            return stop(status);
         }
         if (int s = poll(control)) {
             return stop(s);
         }
         if ((status = passes.extract(&d_back->input, binary, rel, d_out, d_stats, extract_blocks, &d_back->flags))) {
-            return status;
+            return stop(status);
         }
         ctx->launches += 4;
     }
@@ -699,7 +699,7 @@ int correlate(spk_context* ctx, const spk_correlation_spec* spec_ptr, const E* e
         }
         d_mask = static_cast<std::uint8_t*>(device_buffer(ctx, "corr.mask", mask_count, status));
         if (!d_mask) {
-            return status;
+            return stop(status);
         }
         mask_kernel<<<grid_blocks(static_cast<long long>(mask_count), threads), threads, 0, st>>>(
             d_out, padded[0], padded[1], padded[2], delta[0], delta[1], delta[2], mask_request->shape[0],
