@@ -27,6 +27,7 @@ struct spk_context {
     struct Buffer {
         void* ptr {};
         std::size_t bytes {};
+        std::size_t counted {};  // against the cap
     };
     std::map<std::string, Buffer> device_buffers;
     std::map<std::string, Buffer> host_buffers;  // pinned staging
@@ -89,14 +90,17 @@ inline void* device_alloc(spk_context* ctx, std::size_t bytes)
 // Grows (never shrinks) a named device buffer; returns nullptr on failure.
 // These buffers are what the context's cap is about; blocks kept for the next
 // session take no room from it, and go where both would exceed it.  (An open
-// session's kernel data, take_block, lies outside the cap.)
-inline void* device_buffer(spk_context* ctx, const std::string& name, std::size_t bytes, int& status)
+// session's kernel data, take_block, lies outside the cap, and so do `uncounted`
+// bytes of a buffer: a call's bookkeeping.)
+inline void* device_buffer(spk_context* ctx, const std::string& name, std::size_t bytes, int& status,
+                           std::size_t uncounted = 0)
 {
     auto& b = ctx->device_buffers[name];
     if (b.bytes >= bytes && b.ptr) {
         return b.ptr;
     }
-    const std::uint64_t next = ctx->bytes_in_use - b.bytes + bytes;
+    const std::size_t counted = bytes - uncounted;
+    const std::uint64_t next = ctx->bytes_in_use - b.counted + counted;
     if (ctx->cap_bytes && next > ctx->cap_bytes) {
         status = kMemoryLimit;
         return nullptr;
@@ -106,7 +110,7 @@ inline void* device_buffer(spk_context* ctx, const std::string& name, std::size_
     }
     if (b.ptr) {
         cudaFree(b.ptr);
-        ctx->bytes_in_use -= b.bytes;
+        ctx->bytes_in_use -= b.counted;
         b = {};
     }
     void* p = device_alloc(ctx, bytes);
@@ -116,7 +120,8 @@ inline void* device_buffer(spk_context* ctx, const std::string& name, std::size_
     }
     b.ptr = p;
     b.bytes = bytes;
-    ctx->bytes_in_use += bytes;
+    b.counted = counted;
+    ctx->bytes_in_use += counted;
     return p;
 }
 
@@ -127,7 +132,7 @@ inline void drop_buffers(spk_context* ctx, std::initializer_list<const char*> na
         const auto it = ctx->device_buffers.find(name);
         if (it != ctx->device_buffers.end()) {
             cudaFree(it->second.ptr);
-            ctx->bytes_in_use -= it->second.bytes;
+            ctx->bytes_in_use -= it->second.counted;
             ctx->device_buffers.erase(it);
         }
     }

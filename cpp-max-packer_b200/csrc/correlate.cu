@@ -568,14 +568,17 @@ int correlate(spk_context* ctx, const spk_correlation_spec* spec_ptr, const E* e
     const std::size_t result_bytes = mask_request ? mask_count : out_bytes;
     // The inputs side by side, and the small results in front of the large one:
     // small calls then copy once each way.
-    const std::size_t ker_at = (env_count * sizeof(E) + 255) / 256 * 256;
+    const std::size_t ker_at = env_count * sizeof(E);
     constexpr std::size_t out_at = (sizeof(Readback) + 255) / 256 * 256;
     auto* d_in = static_cast<std::uint8_t*>(device_buffer(ctx, "corr.in", ker_at + ker_count, status));
-    auto* d_back = static_cast<Readback*>(device_buffer(ctx, "corr.out", out_at + out_bytes, status));
-    auto* d_stats = static_cast<ExtractStats*>(
-        device_buffer(ctx, "corr.stats", extract_blocks * sizeof(ExtractStats), status));
-    auto* d_partial = static_cast<Compensated2*>(
-        device_buffer(ctx, "corr.partial", (validate_blocks + 8 * kProbeSplit) * sizeof(Compensated2), status));
+    auto* d_back = static_cast<Readback*>(device_buffer(ctx, "corr.out", out_at + out_bytes, status, out_at));
+    // The checks' sums (up to 100 KB) lie outside the cap: the host holds no
+    // others, and a call that fits without them is not refused for them.
+    const std::size_t stats_bytes = extract_blocks * sizeof(ExtractStats);
+    const std::size_t partial_bytes = (validate_blocks + 8 * kProbeSplit) * sizeof(Compensated2);
+    auto* d_stats = static_cast<ExtractStats*>(device_buffer(ctx, "corr.stats", stats_bytes, status, stats_bytes));
+    auto* d_partial =
+        static_cast<Compensated2*>(device_buffer(ctx, "corr.partial", partial_bytes, status, partial_bytes));
     const bool small_in = ker_at + ker_count <= kEarlyResult;
     const std::size_t early_bytes = result_bytes <= kEarlyResult ? result_bytes : 0;
     auto* back = static_cast<Readback*>(host_buffer(ctx, "corr.back", out_at + early_bytes, status));

@@ -1,7 +1,8 @@
 """A correlation that is refused after its work was queued (here by the
 context's memory cap, at the mask's buffer) returns with nothing in flight: its
 inputs are copied from the context's pinned buffer, which the next call
-overwrites."""
+overwrites.  A cap that holds two transform grids, the inputs and the outputs
+refuses nothing: the checks' bookkeeping lies outside it."""
 
 import ctypes
 
@@ -43,3 +44,21 @@ def test_refused_call_leaves_nothing_in_flight(precision):
             assert refused.code == "CORRELATION_MEMORY_LIMIT"
             assert idle
             assert np.array_equal(mask(ctx, legal).mask, want)
+
+
+@pytest.mark.parametrize("es,ks,grid", [((12, 10, 11), (4, 3, 5), (15, 12, 15)), ((20, 24, 22), (5, 6, 4), (24, 30, 25)),
+                                        ((1, 1, 1), (1, 1, 1), (2, 2, 2))])
+@pytest.mark.parametrize("precision", ["FP64", "FP32"])
+def test_a_cap_of_two_grids_inputs_and_outputs_suffices(es, ks, grid, precision):
+    compute = package("compute")
+    rng = np.random.default_rng(5)
+    env = (rng.random(int(np.prod(es))) < 0.2).astype(np.uint8)
+    ker = np.ones(int(np.prod(ks)), np.uint8)
+    cells = int(np.prod([e + k - 1 for e, k in zip(es, ks)]))
+    cap = 2 * int(np.prod(grid)) * (16 if precision == "FP64" else 8) + env.size + ker.size + 8 * cells
+    # Per-block sums of the outputs' checks: 24 bytes for each 256 of them.
+    cap += 24 * -(-cells // 256) + 32
+    with compute.Context(0, cap) as ctx:
+        got = compute.correlate_binary(compute.CorrelationSpec(es, ks), env, ker, precision=getattr(compute, precision),
+                                       context=ctx)
+        assert not isinstance(got, compute.CorrelationFailure), got
