@@ -9,9 +9,10 @@
 // both spectra through Hermitian symmetry, W = E^ conj(K^) is formed, and one
 // inverse 3D FFT (scaled 1/N) yields the correlation in the real part; the
 // imaginary part must stay below the reference's tolerance.  The last pass
-// applies the reference's per-cell checks (correlation.cpp:494-540); input validity and masses (:316-365) and the 8
-// direct probes (:542-577) are reduced on the device beside it, from the copies
-// of the inputs that the transform reads.
+// applies the reference's per-cell checks (correlation.cpp:494-540); input
+// validity and masses (:316-365) and the 8 direct probes (:542-577) are reduced
+// on the device beside it, from the copies of the inputs that the transform
+// reads.
 
 #include <cuda_runtime.h>
 
@@ -502,7 +503,6 @@ int correlate(spk_context* ctx, const spk_correlation_spec* spec_ptr, const E* e
     using C = cplx_t<T>;
     const std::uint64_t grid_bytes = grid * sizeof(C);
     const std::uint64_t out_bytes = padded_count * sizeof(double);
-    const int extract_threads = 256;
     int extract_blocks;
     if constexpr (staged) {
         extract_blocks = stages.blocks();

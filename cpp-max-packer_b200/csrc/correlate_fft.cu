@@ -355,8 +355,8 @@ __global__ void __launch_bounds__(kMaxThreads<CLASS>, kMinPairBlocks<CLASS>)
     }
 }
 
-// x transform back of the output rows and their checks.  A block takes `per` consecutive groups of rows,
-// so that blocks are in index order.
+// x transform back of the output rows and their checks.  A block takes `per`
+// consecutive groups of rows, so that blocks are in index order.
 template <int CLASS>
 __global__ void __launch_bounds__(kMaxThreads<CLASS>, kMinBlocks<CLASS>)
     rows_extract_kernel(const C* __restrict__ z, AxisPlan p, int Ly, int Lz,
@@ -438,12 +438,16 @@ int CorrelationPasses::forward(const E* env, const std::uint8_t* ker) const
     const int rows = fill_y * fill_z, G = kLines;
     const AxisPlan &px = plan[0], &py = plan[1];
     int status = with_class(px, [&](auto c) {
-        return launch<rows_forward_kernel<E, decltype(c)::value>>(dim3((rows + G - 1) / G), block_threads(px), row_bytes(px), stream, z, px, py.L, fill_y, rows, roots[0], shape, env, ker);
+        return launch<rows_forward_kernel<E, decltype(c)::value>>(dim3((rows + G - 1) / G), block_threads(px),
+                                                                  row_bytes(px), stream, z, px, py.L, fill_y, rows,
+                                                                  roots[0], shape, env, ker);
     });
     if (status == kOk) {
         status = with_class(py, [&](auto c) {
-        return launch<columns_kernel<false, decltype(c)::value>>(dim3((px.L + G - 1) / G, fill_z), block_threads(py), column_bytes(py, 1), stream, z, px.L, py, plan[2].L, 0, fill_y, roots[1]);
-    });
+            return launch<columns_kernel<false, decltype(c)::value>>(dim3((px.L + G - 1) / G, fill_z),
+                                                                     block_threads(py), column_bytes(py, 1), stream, z,
+                                                                     px.L, py, plan[2].L, 0, fill_y, roots[1]);
+        });
     }
     return status;
 }
@@ -454,12 +458,16 @@ int CorrelationPasses::multiply() const
     const AxisPlan &px = plan[0], &py = plan[1], &pz = plan[2];
     const double scale = 1.0 / (static_cast<double>(px.L) * py.L * pz.L);
     int status = with_class(pz, [&](auto c) {
-        return launch<pairs_kernel<decltype(c)::value>>(dim3((px.L / 2 + G) / G, py.L), block_threads(pz), column_bytes(pz, 2), stream, z, px.L, py.L, pz, fill_z, roots[2], scale);
+        return launch<pairs_kernel<decltype(c)::value>>(dim3((px.L / 2 + G) / G, py.L), block_threads(pz),
+                                                        column_bytes(pz, 2), stream, z, px.L, py.L, pz, fill_z,
+                                                        roots[2], scale);
     });
     if (status == kOk) {
         status = with_class(py, [&](auto c) {
-        return launch<columns_kernel<true, decltype(c)::value>>(dim3((px.L + G - 1) / G, shape.out[2]), block_threads(py), column_bytes(py, 1), stream, z, px.L, py, pz.L, 1 - shape.ker[2], py.L, roots[1]);
-    });
+            return launch<columns_kernel<true, decltype(c)::value>>(
+                dim3((px.L + G - 1) / G, shape.out[2]), block_threads(py), column_bytes(py, 1), stream, z, px.L, py,
+                pz.L, 1 - shape.ker[2], py.L, roots[1]);
+        });
     }
     return status;
 }
@@ -472,13 +480,15 @@ int CorrelationPasses::extract_blocks() const
 }
 
 int CorrelationPasses::extract(const InputStats* input, bool binary, double rel, double* out, ExtractStats* stats,
-                                  int blocks, OutputFlags* flags) const
+                               int blocks, OutputFlags* flags) const
 {
     const AxisPlan& px = plan[0];
     const long long groups = (static_cast<long long>(shape.out[1]) * shape.out[2] + kLines - 1) / kLines;
     const int per = static_cast<int>((groups + blocks - 1) / blocks);
     return with_class(px, [&](auto c) {
-        return launch<rows_extract_kernel<decltype(c)::value>>(dim3(blocks), block_threads(px), row_bytes(px), stream, z, px, plan[1].L, plan[2].L, roots[0], shape, binary ? 1 : 0, rel, input, per, out, stats, flags);
+        return launch<rows_extract_kernel<decltype(c)::value>>(
+            dim3(blocks), block_threads(px), row_bytes(px), stream, z, px, plan[1].L, plan[2].L, roots[0], shape,
+            binary ? 1 : 0, rel, input, per, out, stats, flags);
     });
 }
 

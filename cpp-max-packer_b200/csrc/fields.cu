@@ -510,7 +510,6 @@ __global__ void fill_kernel(const RasterItem single, const RasterItem* __restric
     }
 }
 
-// out[t] over `req` = OR over stencil deltas d of seed(raw[t - d]) inside `raw`.
 // A sub-box [lo, lo + extent) of a window (cell offsets from its first
 // cell); the box kernels visit its cells only.
 struct CellBox {
@@ -538,6 +537,8 @@ struct FewOffsets {
     signed char at[kFewOffsets][3];
 };
 
+// out[t] over `req` = OR over stencil deltas d of seed(raw[t - d]) inside `raw`;
+// with counts, the cells are added to them as well.
 __global__ void dilate_kernel(const std::uint8_t* __restrict__ raw, FieldWindow rw,
                               const __grid_constant__ FewOffsets few, const int* __restrict__ stencil,
                               int stencil_count, int invert, std::uint8_t* __restrict__ out, FieldWindow req,
@@ -593,17 +594,6 @@ __global__ void occupancy_box_kernel(const std::uint8_t* __restrict__ mask, cons
         box_cell(box, i, c);
         const long long at = c[0] + static_cast<long long>(sx) * (c[1] + static_cast<long long>(sy) * c[2]);
         occ[at] = (mask[at] != 0 || counts[at] != 0) ? 1 : 0;
-    }
-}
-
-__global__ void stamp_kernel(std::uint32_t* __restrict__ counts, const std::uint8_t* __restrict__ placed, long long n,
-                             int direction)
-{
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        if (placed[i]) {
-            counts[i] += direction > 0 ? 1u : static_cast<std::uint32_t>(-1);
-        }
     }
 }
 
@@ -1122,13 +1112,6 @@ int box_mask(spk_context* ctx, const double* dims, double clearance, const Field
     box_mask_kernel<<<blocks_for(n, 256), 256, 0, ctx->stream>>>(d_axes, d_axes + w.shape[0],
                                                                  d_axes + w.shape[0] + w.shape[1], w.shape[0],
                                                                  w.shape[1], w.shape[2], d_mask);
-    ctx->launches++;
-    return cudaGetLastError() == cudaSuccess ? kOk : kCuda;
-}
-
-int stamp(spk_context* ctx, std::uint32_t* d_counts, const std::uint8_t* d_placed, long long n, int direction)
-{
-    stamp_kernel<<<blocks_for(n, 256), 256, 0, ctx->stream>>>(d_counts, d_placed, n, direction);
     ctx->launches++;
     return cudaGetLastError() == cudaSuccess ? kOk : kCuda;
 }

@@ -336,9 +336,10 @@ int copy_to_host(spk_context* ctx, void* dst, const void* d_src, std::size_t byt
         const auto issue = [&] {
             while (issued < c.count &&
                    (issued < c.slots || c.finished[issued - c.slots].load(std::memory_order_acquire))) {
+                const char* from = static_cast<const char*>(d_src) + issued * kSlotBytes;
                 if (ok &&
-                    (cudaMemcpyAsync(slots.slot[issued % c.slots], static_cast<const char*>(d_src) + issued * kSlotBytes,
-                                     c.size(issued), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                    (cudaMemcpyAsync(slots.slot[issued % c.slots], from, c.size(issued), cudaMemcpyDeviceToHost, st) !=
+                         cudaSuccess ||
                      cudaEventRecord(ctx->copy_events[issued % c.slots], st) != cudaSuccess)) {
                     broken();
                 }
@@ -432,7 +433,8 @@ int copy_to_device(spk_context* ctx, void* d_dst, const void* src, std::size_t b
                     continue;
                 }
                 if (arrived < issued) {
-                    const cudaError_t state = ok ? cudaEventQuery(ctx->copy_events[arrived % c.slots]) : cudaErrorUnknown;
+                    const cudaError_t state =
+                        ok ? cudaEventQuery(ctx->copy_events[arrived % c.slots]) : cudaErrorUnknown;
                     if (state != cudaErrorNotReady) {
                         if (ok && state != cudaSuccess) {
                             broken();

@@ -19,10 +19,10 @@ namespace spk {
 // The slots (16 of 512 KB at most) and the helpers belong to the process:
 // pinning costs about a millisecond per megabyte and a thread started per copy
 // about 200 us around its start and end, which every context or copy would pay
-// anew.  The slots are pinned once the copies made have earned that.  Any number of contexts and threads may copy at once: a
-// copy checks out the slots that are free, or takes the plain way where none
-// is, and gets the helpers that are idle.  The last context to go gives all of
-// it back.
+// anew.  The slots are pinned once the copies made have earned that.  Any number
+// of contexts and threads may copy at once: a copy checks out the slots that are
+// free, or takes the plain way where none is, and gets the helpers that are idle.
+// The last context to go gives all of it back.
 int copy_to_host(spk_context* ctx, void* dst, const void* d_src, std::size_t bytes);
 
 // The other way, queued on the context's stream; the source may be reused on

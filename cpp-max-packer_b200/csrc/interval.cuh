@@ -73,22 +73,8 @@ SPK_HD double f_from_bits(std::uint64_t b)
 
 SPK_HD bool f_finite(double v) { return (f_bits(v) & 0x7ff0000000000000ULL) != 0x7ff0000000000000ULL; }
 
-// IEEE nextafter(v, -inf) / nextafter(v, +inf) for finite v, from the bit
-// representation (the next representable binary64 value in that direction).
-SPK_HD double next_down(double v)
-{
-    if (v != v) {
-        return v;
-    }
-    const std::uint64_t b = f_bits(v);
-    if ((b & 0x7fffffffffffffffULL) == 0) {
-        return f_from_bits(0x8000000000000001ULL);  // -denorm_min
-    }
-    if (b >> 63) {
-        return (b & 0x7fffffffffffffffULL) == 0x7ff0000000000000ULL ? v : f_from_bits(b + 1);
-    }
-    return f_from_bits(b - 1);
-}
+// IEEE nextafter(v, +inf) from the bit representation (the next representable
+// binary64 value in that direction).
 SPK_HD double next_up(double v)
 {
     if (v != v) {
@@ -116,7 +102,7 @@ struct Interval {
 
 SPK_HD Interval point_interval(double v) { return { v, v, f_finite(v) }; }
 
-// next_down and next_up of a finite v.  Like the interval operations below
+// The representable values next below and above a finite v.  Like the interval operations below
 // without branches: neighbouring threads' signs differ, and a branch per bound
 // cost the device more than the operations themselves.
 SPK_HD double finite_down(double v)

@@ -25,8 +25,8 @@ constexpr int kColumnBlocks = Plan<L1>::R1 > 24 ? 1 : 1024 / (kColumns * Plan<L1
 // ROW: the row length L0 where it equals L1 (strides are then immediate
 // offsets, which frees registers and issue slots), else 0.
 template <int L1, int ROW>
-__global__ void __launch_bounds__(kColumns* Plan<L1>::T, kColumnBlocks<L1>) pass_b1_kernel(const __grid_constant__ PassBatch batch,
-                                                                        const float2* __restrict__ roots)
+__global__ void __launch_bounds__(kColumns* Plan<L1>::T, kColumnBlocks<L1>)
+    pass_b1_kernel(const __grid_constant__ PassBatch batch, const float2* __restrict__ roots)
 {
     using P = Plan<L1>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -77,9 +77,9 @@ __global__ void __launch_bounds__(kColumns* Plan<L1>::T, kColumnBlocks<L1>) pass
 }
 
 template <int L1, int ROW>
-__global__ void __launch_bounds__(kColumns* Plan<L1>::T, kColumnBlocks<L1>) forward_y_kernel(float2* __restrict__ planes, int row_length, int rows,
-                                                                          const float2* __restrict__ roots,
-                                                                          const EdtBox* __restrict__ region)
+__global__ void __launch_bounds__(kColumns* Plan<L1>::T, kColumnBlocks<L1>)
+    forward_y_kernel(float2* __restrict__ planes, int row_length, int rows, const float2* __restrict__ roots,
+                     const EdtBox* __restrict__ region)
 {
     using P = Plan<L1>;
     extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -1379,9 +1379,9 @@ int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vect
     // costs little more.  Later rounds visit twice as many planes as the one
     // before.  Planes that heads need, and a step's time by the planes visited
     // first: 24 cuboids on a 66^3 window 2 to 5 of 50 (47 planes 297 us, 15 planes
-    // 278 us); 96 blobs of 52 planes on a 128^3 window 4 to 11 of 80 (45 planes
-    // 1.25 ms, 13 planes 0.90 ms); 32 blobs of 25 planes on a 256^3 window 28 to 31 of
-    // 231 (40 planes; 8 would take three rounds).
+    // 278 us); 32 blobs of 25 planes on a 256^3 window 28 to 31 of 231 (40 planes; 8
+    // would take three rounds).  Requests that are not pruned visit every plane
+    // in the first round.
     int step = INT32_MAX;
     if (goal.prune) {
         int n = 0, range = 0;

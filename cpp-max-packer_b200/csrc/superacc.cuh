@@ -85,13 +85,6 @@ SPK_HD void super_add_at(SuperAcc& a, unsigned long long v, int pos)
     }
 }
 
-SPK_HD void super_merge(SuperAcc& a, const SuperAcc& b)
-{
-    for (int i = 0; i < kSuperLimbs; ++i) {
-        a.limb[i] += b.limb[i];
-    }
-}
-
 // Correctly rounded (nearest, ties to even) binary64 value of the sum.
 SPK_HD double super_round(const SuperAcc& in)
 {
