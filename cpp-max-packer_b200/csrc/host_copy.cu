@@ -191,6 +191,15 @@ void wait_until(const Condition& condition)
     }
 }
 
+// Whether CUDA knows the memory: the DMA reaches pinned or managed pages itself
+// (STL files of 33 and 100 MB into pinned memory 0.65 and 1.9 ms, 0.93 and 2.9
+// through slots).
+bool registered(const void* at)
+{
+    cudaPointerAttributes a {};
+    return cudaPointerGetAttributes(&a, at) == cudaSuccess && a.type != cudaMemoryTypeUnregistered;
+}
+
 // Whether more than a sixteenth of `bytes` from `at` on lies in pages that were
 // never touched, as far as both ends tell: from there on the slots' 10 us per MB
 // more are less than the 180 us per MB that they save on those pages.
@@ -311,8 +320,10 @@ int copy_to_host(spk_context* ctx, void* dst, const void* d_src, std::size_t byt
 {
     cudaStream_t st = ctx->stream;
     bool ok = true;
-    const bool fresh = untouched(dst, bytes);
-    const bool staged = fresh || bytes <= kSmallBytes || (bytes >= kHelpedBytes && most_helpers() > 1);
+    const bool pageable = bytes && !registered(dst);
+    const bool fresh = pageable && untouched(dst, bytes);
+    const bool staged =
+        fresh || (pageable && (bytes <= kSmallBytes || (bytes >= kHelpedBytes && most_helpers() > 1)));
     Slots slots(ctx, staged ? std::min((bytes + kSlotBytes - 1) / kSlotBytes, kMaxSlots) : 0,
                 staged ? mega(bytes) * (fresh ? kSavedUntouched : kSavedTouched) : 0.0);
     if (!slots.usable()) {
@@ -391,7 +402,7 @@ int copy_to_device(spk_context* ctx, void* d_dst, const void* src, std::size_t b
 {
     cudaStream_t st = ctx->stream;
     bool ok = true;
-    if (bytes < kSourceBytes || most_helpers() < 2) {
+    if (bytes < kSourceBytes || most_helpers() < 2 || registered(src)) {
         ok = cudaMemcpyAsync(d_dst, src, bytes, cudaMemcpyHostToDevice, st) == cudaSuccess;
     }
     else {

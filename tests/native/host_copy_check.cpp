@@ -58,6 +58,7 @@ std::atomic<long long> pinned { 0 };
 std::atomic<int> pin_calls { 0 };
 bool pin_fails = false;
 std::size_t largest_dma = 0;
+const void* known_to_cuda = nullptr;  // pinned by the caller
 std::function<void()> on_synchronize;
 
 int failures = 0;
@@ -152,6 +153,12 @@ cudaError_t cudaFreeHost(void* p)
     return cudaSuccess;
 }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p)
+{
+    *a = {};
+    a->type = p == known_to_cuda ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;
+    return cudaSuccess;
+}
 cudaError_t cudaMalloc(void**, size_t) { return cudaErrorMemoryAllocation; }
 cudaError_t cudaFree(void*) { return cudaSuccess; }
 }
@@ -223,11 +230,12 @@ void ways()
     Context c;
     check(round_trip(c, 64 * MB, 1), "a copy that earns both chunks of slots");
     const bool helped = spk::most_helpers() > 1;
-    const auto staged = [&](std::size_t n, bool to_device, bool touched) {
+    const auto staged = [&](std::size_t n, bool to_device, bool touched, bool known = false) {
         char* host = static_cast<char*>(mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0));
         if (touched) {
             std::memset(host, 1, n);
         }
+        known_to_cuda = known ? host : nullptr;
         std::vector<char> device(n, 2);
         largest_dma = 0;
         const int status = to_device ? spk::copy_to_device(&c.ctx, device.data(), host, n)
@@ -249,6 +257,8 @@ void ways()
     for (std::size_t mb : { 8, 11, 12, 16, 50 }) {
         check(staged(mb * MB, false, true) == helped, "larger copies take the slots where there are helpers");
         check(staged(mb * MB, true, true) == (helped && mb >= 12), "and larger sources");
+        check(!staged(mb * MB, false, true, true) && !staged(mb * MB, true, true, true),
+              "pinned memory takes the plain way");
     }
 }
 
@@ -287,6 +297,26 @@ void pins()
         check(pin_calls == 2, "one large copy earns both at once");
     }
     check(pinned == 0, "and gives them back");
+}
+
+void pinned_by_the_caller()
+{
+    Context c;
+    check(round_trip(c, 64 * MB, 1), "a copy that earns the slots");
+    for (std::size_t n : { 700 * KB, 3 * MB / 2, 3 * MB, 9 * MB, 40 * MB }) {
+        const auto want = pattern(n, 2);
+        std::vector<char> to(n);
+        known_to_cuda = to.data();
+        largest_dma = 0;
+        check(spk::copy_to_host(&c.ctx, to.data(), want.data(), n) == spk::kOk && to == want && largest_dma == n,
+              "a pinned destination gets one DMA");
+        known_to_cuda = want.data();
+        largest_dma = 0;
+        check(spk::copy_to_device(&c.ctx, to.data(), want.data(), n) == spk::kOk, "a copy to the device");
+        cudaStreamSynchronize(c.ctx.stream);
+        check(to == want && largest_dma == n, "a pinned source too");
+        known_to_cuda = nullptr;
+    }
 }
 
 void no_slots()
@@ -394,6 +424,9 @@ int main(int, char** argv)
     }
     else if (which == "pins") {
         pins();
+    }
+    else if (which == "pinned_by_the_caller") {
+        pinned_by_the_caller();
     }
     else if (which == "no_slots") {
         no_slots();

@@ -26,7 +26,7 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("check", ["sizes", "ways", "pins", "no_slots", "threads", "helpers_live", "failing_copy"])
+@pytest.mark.parametrize("check", ["sizes", "ways", "pins", "pinned_by_the_caller", "no_slots", "threads", "helpers_live", "failing_copy"])
 def test_copies(program, check):
     out = subprocess.run([program, check], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0, out.stdout + out.stderr
