@@ -125,6 +125,13 @@ inline void* device_buffer(spk_context* ctx, const std::string& name, std::size_
     return p;
 }
 
+// What a capped context has left for a named buffer, its present size included.
+inline std::uint64_t room_for(const spk_context* ctx, const char* name)
+{
+    const auto it = ctx->device_buffers.find(name);
+    return ctx->cap_bytes - ctx->bytes_in_use + (it == ctx->device_buffers.end() ? 0 : it->second.counted);
+}
+
 // Gives named device buffers back.
 inline void drop_buffers(spk_context* ctx, std::initializer_list<const char*> names)
 {

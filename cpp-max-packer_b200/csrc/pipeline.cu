@@ -1029,9 +1029,8 @@ int Pipeline::run_planes(const std::vector<PlaneWork>& work, PassMode mode, bool
             int per_launch = static_cast<int>(
                 std::min<std::size_t>(std::max<std::size_t>(kInterBytes / bytes, 1), static_cast<std::size_t>(n)));
             if (ctx_->cap_bytes) {  // half of what is left: placements need theirs
-                const std::uint64_t left = ctx_->cap_bytes - ctx_->bytes_in_use;
-                per_launch = static_cast<int>(
-                    std::max<std::uint64_t>(1, std::min<std::uint64_t>(per_launch, left / 2 / bytes)));
+                per_launch = static_cast<int>(std::max<std::uint64_t>(
+                    1, std::min<std::uint64_t>(per_launch, room_for(ctx_, "pipe.inter") / 2 / bytes)));
             }
             float2* inter = nullptr;
             while (!inter) {  // under a device-memory cap, fewer orientations per launch
@@ -1335,7 +1334,7 @@ int Pipeline::ordinary_pages(const std::vector<PageRequest>& requests, std::vect
             return status;
         }
         const std::uint64_t chunk_bytes = static_cast<std::uint64_t>(R) * (kKeyCapacity + per) * 8;
-        while (chunks > 1 && chunks * chunk_bytes > (ctx_->cap_bytes - ctx_->bytes_in_use) / 4) {
+        while (chunks > 1 && chunks * chunk_bytes > room_for(ctx_, "pipe.keys") / 4) {
             chunks /= 2;
         }
     }

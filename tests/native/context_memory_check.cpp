@@ -96,6 +96,8 @@ int main()
         check(used == 60 * MB, "a block past the cap is not kept");
         check(!spk::device_buffer(&ctx, "b", 121 * MB, status) && status == spk::kMemoryLimit && used == 60 * MB,
               "a buffer past the cap is refused");
+        check(spk::room_for(&ctx, "b") == 120 * MB && spk::room_for(&ctx, "c") == 60 * MB,
+              "room for a buffer counts what it has");
         spk::drop_buffers(&ctx, { "b" });
     }
     std::printf(failures ? "%d failed\n" : "ok\n", failures);
