@@ -27,7 +27,7 @@ constexpr std::size_t kChunkSlots = 8;  // slots pinned at once
 constexpr std::size_t kMaxSlots = 16;
 // Which way is the fastest depends on the size and on what the CPU last did
 // with the destination's pages: medians in us, 200 to 300 us apart, so that
-// helpers sleep in between and cost up to 300 us to wake (two boxes).
+// helpers sleep in between and cost up to 300 us to wake (two machines).
 //
 //   MB to the host               0.5    1  1.5    2    4    8   10   16    33
 //   touched, not lately  plain    50   84  116  139  249  484  576  866  1634
